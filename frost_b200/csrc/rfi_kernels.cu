@@ -25,6 +25,7 @@
 #include <cuda_runtime.h>
 
 #include "common.hpp"
+#include "rfi_columns.cuh"
 #include "rfi_kernels.hpp"
 #include "rfi_stage.cuh"
 
@@ -181,125 +182,6 @@ __global__ void k_sample_rows(Dims d, const uint8_t* __restrict__ raw, float* __
         dst[c] = rd<D>(in, c);
 }
 
-// Recursive median-of-5 over m = 5^k values streamed in order: the same
-// groups of five, level by level, as the batch remedian in
-// lib/cpu/spectra_cpu.cpp:43-69.
-struct Remedian {
-    float buf[5][5];
-    int cnt[5];
-    int depth;
-    float result;
-
-    __device__ void init(int levels) {
-        depth = levels;
-        for (int l = 0; l < 5; ++l)
-            cnt[l] = 0;
-        result = 0.0F;
-    }
-    __device__ void push(float x) {
-        int l = 0;
-        while (true) {
-            if (l == depth) {
-                result = x;
-                return;
-            }
-            buf[l][cnt[l]++] = x;
-            if (cnt[l] < 5)
-                return;
-            cnt[l] = 0;
-            x      = median5(buf[l][0], buf[l][1], buf[l][2], buf[l][3], buf[l][4]);
-            ++l;
-        }
-    }
-};
-
-__global__ void k_bandpass(Dims d, const float* __restrict__ samples, float* __restrict__ loc_out,
-                           float* __restrict__ scale_out, float* __restrict__ inv_out,
-                           uint32_t* __restrict__ unmeasured) {
-    const uint64_t c = blockIdx.x * static_cast<uint64_t>(blockDim.x) + threadIdx.x;
-    const uint64_t w = blockIdx.y;
-    if (c >= d.nchans)
-        return;
-    const uint64_t b   = window_begin(w, d.window);
-    const uint64_t len = window_end(w, d) - b;
-    const uint64_t m   = largest_power_of_five_leq(len < kMaxBandpassRows ? len : kMaxBandpassRows);
-    int levels         = 0;
-    for (uint64_t p = m; p > 1; p /= 5)
-        ++levels;
-    const uint64_t n = d.nchans;
-    const float* v   = samples + w * kMaxBandpassRows * n + c;
-
-    // Level: remedian over the sampled rows; scale: remedian of |x - level|
-    // times 1.4826 (lib/cpu/spectra_cpu.cpp:73-130).
-    Remedian r;
-    r.init(levels);
-    for (uint64_t i = 0; i < m; ++i)
-        r.push(v[i * n]);
-    const float level = r.result;
-    r.init(levels);
-    for (uint64_t i = 0; i < m; ++i)
-        r.push(fabsf(v[i * n] - level));
-    const float rms = r.result * kMadToStd;
-
-    // Clipped refinement in double (lib/cpu/bandpass_kernels.hpp:17-76).
-    float lo = v[0], hi = v[0];
-    for (uint64_t i = 1; i < m; ++i) {
-        lo = smin(lo, v[i * n]);
-        hi = smax(hi, v[i * n]);
-    }
-    const uint64_t o = w * n + c;
-    if (!(hi > lo)) {
-        loc_out[o]   = lo;
-        scale_out[o] = 0.0F;
-        inv_out[o]   = 0.0F;
-        atomicAdd(&unmeasured[c], 1U);
-        return;
-    }
-    double centre = level;
-    double s      = rms;
-    const double dm = static_cast<double>(m);
-    if (!(s > 0.0)) {
-        double mean = 0.0;
-        for (uint64_t i = 0; i < m; ++i)
-            mean += v[i * n];
-        mean /= dm;
-        double ss = 0.0;
-        for (uint64_t i = 0; i < m; ++i)
-            ss += (v[i * n] - mean) * (v[i * n] - mean);
-        s = sqrt(ss / dm);
-    }
-    for (int it = 0; it < kClipIterations; ++it) {
-        const double cut = kClipSigma * s;
-        double count = 0.0, sum = 0.0;
-        for (uint64_t i = 0; i < m; ++i) {
-            const double dv = v[i * n] - centre;
-            if (fabs(dv) <= cut) {
-                count += 1.0;
-                sum += dv;
-            }
-        }
-        if (count < 2.0)
-            break;
-        const double shift = sum / count;
-        double ss          = 0.0;
-        for (uint64_t i = 0; i < m; ++i) {
-            const double dv = v[i * n] - centre;
-            if (fabs(dv) <= cut)
-                ss += (dv - shift) * (dv - shift);
-        }
-        const double clipped = sqrt(ss / count);
-        if (!(clipped > 0.0))
-            break;
-        centre += shift;
-        s = clipped;
-    }
-    const float fl = static_cast<float>(centre);
-    const float fs = static_cast<float>(s);
-    loc_out[o]     = fl;
-    scale_out[o]   = fs;
-    inv_out[o]     = 1.0F / fs;
-}
-
 // The remedian is a fixed tree (medians of five consecutive values, level by
 // level), so its groups are independent: k_remedian evaluates it in
 // parallel. One CTA covers 32 channels (a lane each) of one window; each
@@ -447,107 +329,99 @@ __global__ void __launch_bounds__(32 * kRemedianWarps)
 }
 
 // The clipped refinement of the bandpass (lib/cpu/bandpass_kernels.hpp:17-76)
-// after the two remedian passes, with the sampled rows streamed through
-// shared memory (rfi_stage.cuh), one thread per channel of a 128-channel
-// segment. Every pass over the rows is one staged sweep; the block runs the
-// optional passes (mean fallback, clip iterations) when any of its channels
-// needs them, and each channel updates only while its own sequence of steps
-// is still running, so every channel takes exactly the steps of the direct
-// kernel above. A flat channel (every sampled value equal) keeps its first
+// after the two remedian passes: a lane per channel, a warp (one CTA) per 32
+// channels of a window. Up to six passes over the sampled rows, each one
+// chain of dependent FP64 additions in row order: bound by that chain (8
+// cycles a row) while there are fewer warps than schedulers, so the rows are
+// streamed by the warp itself (rfi_columns.cuh) and everything but the
+// additions is done 16 rows ahead of them. 1024 channels, 2 windows: 172 us
+// (1002 with block-wide staging and one row's loads at a time); 4096
+// channels, 8 windows: 240 us (1056).
+// Each channel updates only while its own sequence of steps is still
+// running, so every channel takes the reference's steps whatever the others
+// of its warp do. A flat channel (every sampled value equal) keeps its first
 // sampled value as its level, as the sequential minimum does.
-constexpr int kBandChans = 128;
-
-__global__ void __launch_bounds__(kBandChans)
-    k_bandpass_staged(Dims d, const float* __restrict__ samples, float* __restrict__ loc_out,
+template <int U>
+__global__ void __launch_bounds__(32)
+    k_bandpass_refine(Dims d, const float* __restrict__ samples, float* __restrict__ loc_out,
                       float* __restrict__ scale_out, float* __restrict__ inv_out,
-                      uint32_t* __restrict__ unmeasured, int seg_bytes, int rows) {
-    extern __shared__ __align__(16) uint8_t stage_buf[];
-    const uint64_t c0  = static_cast<uint64_t>(blockIdx.x) * kBandChans;
+                      uint32_t* __restrict__ unmeasured) {
+    using Reader = cols::Reader<32, U, 32, 4>;
+    __shared__ __align__(16) uint8_t ring[Reader::kBytes];
+    const uint64_t c0  = static_cast<uint64_t>(blockIdx.x) * 32;
     const uint64_t c   = c0 + threadIdx.x;
     const uint64_t w   = blockIdx.y;
     const bool in      = c < d.nchans;
-    const uint64_t b   = window_begin(w, d.window);
-    const uint64_t len = window_end(w, d) - b;
+    const uint64_t len = window_end(w, d) - window_begin(w, d.window);
     const uint64_t m   = largest_power_of_five_leq(len < kMaxBandpassRows ? len : kMaxBandpassRows);
-    const uint64_t n     = d.nchans;
-    const uint64_t pitch = n * sizeof(float);
-    const uint64_t left  = pitch - c0 * sizeof(float);
-    const int copy       = static_cast<int>(left < static_cast<uint64_t>(seg_bytes) ? left : seg_bytes);
-    const int stride     = seg_bytes / static_cast<int>(sizeof(float));
-    const uint8_t* src   = reinterpret_cast<const uint8_t*>(samples + w * kMaxBandpassRows * n + c0);
-    // one sweep over rows 0 .. m-1: f(x, i) per row, in order
+    const uint64_t n   = d.nchans;
+    const Reader rows(ring, reinterpret_cast<const uint8_t*>(samples + w * kMaxBandpassRows * n + c0),
+                      n * sizeof(float), (n - c0) * sizeof(float), m);
+    // one sweep over rows 0 .. m-1: f(nb, x) per batch of rows, in order
     auto sweep = [&](auto&& f) {
-        stage::StagerN<kDeepStages> st(stage_buf, src, pitch, seg_bytes, copy, rows, 0, m);
-        st.start();
-        for (int k = 0; k < st.nblk; ++k) {
-            st.wait(k);
-            const float* buf = reinterpret_cast<const float*>(st.buf(k));
-            const int nr     = st.rows_of(k);
-            const uint64_t i0 = st.t0(k);
-            if (in)
-                for (int r = 0; r < nr; ++r)
-                    f(buf[r * stride + threadIdx.x], i0 + r);
-            st.release(k);
-        }
+        rows.template each<16>([](const uint8_t* row, int lane) { return reinterpret_cast<const float*>(row)[lane]; },
+                               [&](auto nb, const float* x, int, const double2*) { f(nb, x); });
     };
 
-    const uint64_t o   = w * n + c;
-    const float level  = in ? loc_out[o] : 0.0F;
-    const float rms    = in ? scale_out[o] : 0.0F;
-    const bool flat    = in && inv_out[o] != 0.0F;
-    if (in && flat) {
+    const uint64_t o  = w * n + c;
+    const float level = in ? loc_out[o] : 0.0F;
+    const float rms   = in ? scale_out[o] : 0.0F;
+    const bool flat   = in && inv_out[o] != 0.0F;
+    if (flat) {
         loc_out[o]   = samples[w * kMaxBandpassRows * n + c];
         scale_out[o] = 0.0F;
         inv_out[o]   = 0.0F;
         atomicAdd(&unmeasured[c], 1U);
     }
-    bool live       = in && !flat;
-    double centre   = level;
-    double sd       = rms;
-    const double dm = static_cast<double>(m);
+    bool live            = in && !flat;
+    double centre        = level;
+    double sd            = rms;
+    const double dm      = static_cast<double>(m);
     const bool need_mean = live && !(sd > 0.0);
-    if (__syncthreads_or(need_mean)) {
+    if (__any_sync(0xFFFFFFFFU, need_mean)) {
         double mean = 0.0;
-        sweep([&](float x, uint64_t) {
-            if (need_mean)
-                mean += x;
+        sweep([&](auto nb, const float* x) {
+#pragma unroll
+            for (int j = 0; j < nb; ++j)
+                mean += x[j];
         });
         mean /= dm;
         double ss = 0.0;
-        sweep([&](float x, uint64_t) {
-            if (need_mean)
-                ss += (x - mean) * (x - mean);
+        sweep([&](auto nb, const float* x) {
+#pragma unroll
+            for (int j = 0; j < nb; ++j)
+                ss += (x[j] - mean) * (x[j] - mean);
         });
         if (need_mean)
             sd = sqrt(ss / dm);
     }
     for (int it = 0; it < kClipIterations; ++it) {
-        if (!__syncthreads_or(live))
+        if (!__any_sync(0xFFFFFFFFU, live))
             break;
         const double cut = kClipSigma * sd;
         uint32_t kept    = 0; // the count of kept samples (exact as a double)
         double sum       = 0.0;
-        sweep([&](float x, uint64_t) {
-            if (live) {
-                const double dv = x - centre;
-                if (fabs(dv) <= cut) {
-                    ++kept;
-                    sum += dv;
-                }
+        sweep([&](auto nb, const float* x) {
+#pragma unroll
+            for (int j = 0; j < nb; ++j) {
+                const double dv = x[j] - centre;
+                const bool keep = fabs(dv) <= cut;
+                kept += keep ? 1U : 0U;
+                sum += keep ? dv : 0.0; // a sum is never -0, so +0 leaves it as it is
             }
         });
         const double count = static_cast<double>(kept);
         if (live && count < 2.0)
             live = false;
         const double shift = live ? sum / count : 0.0;
-        if (!__syncthreads_or(live))
+        if (!__any_sync(0xFFFFFFFFU, live))
             break;
         double ss = 0.0;
-        sweep([&](float x, uint64_t) {
-            if (live) {
-                const double dv = x - centre;
-                if (fabs(dv) <= cut)
-                    ss += (dv - shift) * (dv - shift);
+        sweep([&](auto nb, const float* x) {
+#pragma unroll
+            for (int j = 0; j < nb; ++j) {
+                const double dv = x[j] - centre;
+                ss += fabs(dv) <= cut ? (dv - shift) * (dv - shift) : 0.0;
             }
         });
         if (live) {
@@ -1908,24 +1782,16 @@ void launch_sample_rows(const Dims& d, const uint8_t* raw, float* samples, cudaS
 
 void launch_bandpass(const Dims& d, const float* samples, float* loc, float* scale, float* inv,
                      uint32_t* unmeasured, cudaStream_t s) {
-    const uint64_t pitch = d.nchans * sizeof(float);
-    if (pitch % 16 != 0 || reinterpret_cast<uintptr_t>(samples) % 16 != 0) {
-        const dim3 grid(grid1(d.nchans, 64), static_cast<unsigned>(d.nwin));
-        k_bandpass<<<grid, 64, 0, s>>>(d, samples, loc, scale, inv, unmeasured);
-    } else {
-        // level and flat flag, then the scale, then the clipped refinement
-        const dim3 rgrid(grid1(d.nchans, 32), static_cast<unsigned>(d.nwin));
-        k_remedian<false><<<rgrid, 32 * kRemedianWarps, 0, s>>>(d, samples, loc, scale, inv);
-        FB_COUNT_LAUNCH();
-        k_remedian<true><<<rgrid, 32 * kRemedianWarps, 0, s>>>(d, samples, loc, scale, inv);
-        FB_COUNT_LAUNCH();
-        const int seg     = static_cast<int>(std::min<uint64_t>(kBandChans * sizeof(float), pitch));
-        const int rows    = std::max(8, 16384 / seg);
-        const size_t smem = kDeepStages * static_cast<size_t>(seg) * rows;
-        const dim3 grid(grid1(d.nchans, kBandChans), static_cast<unsigned>(d.nwin));
-        set_smem(reinterpret_cast<const void*>(&k_bandpass_staged), smem);
-        k_bandpass_staged<<<grid, kBandChans, smem, s>>>(d, samples, loc, scale, inv, unmeasured, seg, rows);
-    }
+    // level and flat flag, then the scale, then the clipped refinement
+    const dim3 grid(grid1(d.nchans, 32), static_cast<unsigned>(d.nwin));
+    k_remedian<false><<<grid, 32 * kRemedianWarps, 0, s>>>(d, samples, loc, scale, inv);
+    FB_COUNT_LAUNCH();
+    k_remedian<true><<<grid, 32 * kRemedianWarps, 0, s>>>(d, samples, loc, scale, inv);
+    FB_COUNT_LAUNCH();
+    if (d.nchans % 4 == 0 && reinterpret_cast<uintptr_t>(samples) % 16 == 0)
+        k_bandpass_refine<16><<<grid, 32, 0, s>>>(d, samples, loc, scale, inv, unmeasured);
+    else
+        k_bandpass_refine<4><<<grid, 32, 0, s>>>(d, samples, loc, scale, inv, unmeasured);
     FB_COUNT_LAUNCH();
 }
 
