@@ -96,10 +96,6 @@ constexpr uint64_t kBitsOf = D == FROST_UINT1 ? 1 : D == FROST_UINT2 ? 2 : D == 
 // channel) loops: the loads are independent, only the sums are sequential.
 constexpr int kBlock = 16;
 
-// Buffers of the per-window sequence kernels' staging: with one or two CTAs
-// per SM, three stages in flight keep enough bytes moving for the chains.
-constexpr int kDeepStages = 4;
-
 // ---- order-exact helpers ------------------------------------------------
 
 // std::min / std::max semantics (first argument kept on ties), which the
@@ -329,39 +325,101 @@ __global__ void __launch_bounds__(32 * kRemedianWarps)
 }
 
 // The clipped refinement of the bandpass (lib/cpu/bandpass_kernels.hpp:17-76)
-// after the two remedian passes: a lane per channel, a warp (one CTA) per 32
-// channels of a window. Up to six passes over the sampled rows, each one
-// chain of dependent FP64 additions in row order: bound by that chain (8
-// cycles a row) while there are fewer warps than schedulers, so the rows are
-// streamed by the warp itself (rfi_columns.cuh) and everything but the
-// additions is done 16 rows ahead of them. 1024 channels, 2 windows: 172 us
-// (1002 with block-wide staging and one row's loads at a time); 4096
-// channels, 8 windows: 240 us (1056).
+// after the two remedian passes: a lane per channel, a CTA per 32 channels
+// of a window. Up to six passes over the sampled rows, each one chain of
+// dependent FP64 additions in row order, streamed as rfi_columns.cuh says.
+// 1024 channels, 2 windows: 122 us (172 with a warp that copies for itself
+// and a loop the compiler orders); 4096 channels, 8 windows: 304 us.
 // Each channel updates only while its own sequence of steps is still
 // running, so every channel takes the reference's steps whatever the others
 // of its warp do. A flat channel (every sampled value equal) keeps its first
 // sampled value as its level, as the sequential minimum does.
-template <int U>
-__global__ void __launch_bounds__(32)
+template <int U, int G> using SampleRing = cols::Ring<32, U, G == 1 ? 64 : 32, 4>;
+
+// The sum over a column, in row order, of d = x - centre where |d| <= cut
+// (SQUARE: of (d - shift)^2 there), and how many they are. A sum from +0 is
+// never -0, so the +0 of a sample that is not kept leaves it as it is.
+template <bool SQUARE, class R>
+__device__ __forceinline__ double clipped_sum(const R& rows, double centre, double cut, double shift, uint32_t& kept) {
+    constexpr int A = cols::kAhead;
+    double sum      = 0.0;
+    uint32_t count  = 0;
+    uint32_t raw[A];          // row j in raw[j % A], read A rows ahead
+    double x[4], d[4], v[2];  // widened 4 rows ahead, differences 3, terms 1
+    uint32_t one[2];
+    auto term = [&](double& t, uint32_t& o, double dv) {
+        if constexpr (SQUARE) {
+            double e;
+            cols::sub(e, dv, shift);
+            cols::mul(e, e, e);
+            asm volatile("{\n\t.reg .pred p;\n\t.reg .f64 a;\n\tabs.f64 a, %1;\n\tsetp.le.f64 p, a, %2;\n\t"
+                         "selp.f64 %0, %3, 0d0000000000000000, p;\n\t}"
+                         : "=d"(t)
+                         : "d"(dv), "d"(cut), "d"(e));
+            o = 1;
+        } else {
+            cols::keep(t, o, dv, cut);
+        }
+    };
+    rows.walk(
+        [&](uint32_t a) {
+#pragma unroll
+            for (int j = 0; j < A; ++j)
+                raw[j] = rows.bits(a + j * R::kPitch, j);
+#pragma unroll
+            for (int j = 0; j < 4; ++j)
+                cols::widen(x[j], __uint_as_float(raw[j]));
+#pragma unroll
+            for (int j = 0; j < 3; ++j)
+                cols::sub(d[j], x[j], centre);
+            term(v[0], one[0], d[0]);
+        },
+        [&](int r, uint32_t a, uint32_t b) {
+#pragma unroll
+            for (int j = 0; j < cols::kBatch; ++j) {
+                cols::add(sum, sum, v[j & 1]);
+                count += one[j & 1];
+                raw[j % A] = rows.bits(j + A < cols::kBatch ? a + (j + A) * R::kPitch
+                                                            : b + (j + A - cols::kBatch) * R::kPitch, r + j + A);
+                cols::sub(d[(j + 3) & 3], x[(j + 3) & 3], centre);
+                term(v[(j + 1) & 1], one[(j + 1) & 1], d[(j + 1) & 3]);
+                cols::widen(x[j & 3], __uint_as_float(raw[(j + 4) % A]));
+            }
+        },
+        [&](int r, uint32_t a) {
+            double dv, t;
+            uint32_t o;
+            cols::widen(dv, __uint_as_float(rows.bits(a, r)));
+            cols::sub(dv, dv, centre);
+            term(t, o, dv);
+            cols::add(sum, sum, t);
+            count += o;
+        });
+    kept = count;
+    return sum;
+}
+
+template <int U, int G>
+__global__ void __launch_bounds__(32 * (G + 1))
     k_bandpass_refine(Dims d, const float* __restrict__ samples, float* __restrict__ loc_out,
                       float* __restrict__ scale_out, float* __restrict__ inv_out,
                       uint32_t* __restrict__ unmeasured) {
-    using Reader = cols::Reader<32, U, 32, 4>;
-    __shared__ __align__(16) uint8_t ring[Reader::kBytes];
-    const uint64_t c0  = static_cast<uint64_t>(blockIdx.x) * 32;
-    const uint64_t c   = c0 + threadIdx.x;
-    const uint64_t w   = blockIdx.y;
-    const bool in      = c < d.nchans;
-    const uint64_t len = window_end(w, d) - window_begin(w, d.window);
-    const uint64_t m   = largest_power_of_five_leq(len < kMaxBandpassRows ? len : kMaxBandpassRows);
-    const uint64_t n   = d.nchans;
-    const Reader rows(ring, reinterpret_cast<const uint8_t*>(samples + w * kMaxBandpassRows * n + c0),
-                      n * sizeof(float), (n - c0) * sizeof(float), m);
-    // one sweep over rows 0 .. m-1: f(nb, x) per batch of rows, in order
-    auto sweep = [&](auto&& f) {
-        rows.template each<16>([](const uint8_t* row, int lane) { return reinterpret_cast<const float*>(row)[lane]; },
-                               [&](auto nb, const float* x, int, const double2*) { f(nb, x); });
+    using R = SampleRing<U, G>;
+    extern __shared__ __align__(16) uint8_t rings[]; // [G][R::kBytes]
+    const bool feeder    = threadIdx.x < 32;
+    const uint64_t first = static_cast<uint64_t>(blockIdx.x) * 32 * G;
+    const uint64_t w     = blockIdx.y;
+    const uint64_t len   = window_end(w, d) - window_begin(w, d.window);
+    const uint64_t m     = largest_power_of_five_leq(len < kMaxBandpassRows ? len : kMaxBandpassRows);
+    const uint64_t n     = d.nchans;
+    auto ring            = [&](int g) {
+        const uint64_t c0 = first + 32 * static_cast<uint64_t>(g);
+        return R(rings + g * R::kBytes, reinterpret_cast<const uint8_t*>(samples + w * kMaxBandpassRows * n + c0),
+                 n * sizeof(float), c0 < n ? (n - c0) * sizeof(float) : 0, m);
     };
+    const uint64_t c = first + threadIdx.x - 32;
+    const bool in    = !feeder && c < n;
+    const R rows     = ring(feeder ? 0 : static_cast<int>(threadIdx.x >> 5U) - 1);
 
     const uint64_t o  = w * n + c;
     const float level = in ? loc_out[o] : 0.0F;
@@ -378,52 +436,40 @@ __global__ void __launch_bounds__(32)
     double sd            = rms;
     const double dm      = static_cast<double>(m);
     const bool need_mean = live && !(sd > 0.0);
-    if (__any_sync(0xFFFFFFFFU, need_mean)) {
-        double mean = 0.0;
-        sweep([&](auto nb, const float* x) {
-#pragma unroll
-            for (int j = 0; j < nb; ++j)
-                mean += x[j];
-        });
-        mean /= dm;
-        double ss = 0.0;
-        sweep([&](auto nb, const float* x) {
-#pragma unroll
-            for (int j = 0; j < nb; ++j)
-                ss += (x[j] - mean) * (x[j] - mean);
-        });
-        if (need_mean)
-            sd = sqrt(ss / dm);
+    const double all     = __longlong_as_double(0x7FF0000000000000LL); // keeps every sample
+    uint32_t kept        = 0;
+    if (__syncthreads_or(need_mean)) {
+        if (feeder) {
+            R::template feed<G>(ring);
+            R::template feed<G>(ring);
+        } else {
+            const double mean = clipped_sum<false>(rows, 0.0, all, 0.0, kept) / dm;
+            const double ss   = clipped_sum<true>(rows, 0.0, all, mean, kept);
+            if (need_mean)
+                sd = sqrt(ss / dm);
+        }
     }
     for (int it = 0; it < kClipIterations; ++it) {
-        if (!__any_sync(0xFFFFFFFFU, live))
+        if (!__syncthreads_or(live))
             break;
         const double cut = kClipSigma * sd;
-        uint32_t kept    = 0; // the count of kept samples (exact as a double)
-        double sum       = 0.0;
-        sweep([&](auto nb, const float* x) {
-#pragma unroll
-            for (int j = 0; j < nb; ++j) {
-                const double dv = x[j] - centre;
-                const bool keep = fabs(dv) <= cut;
-                kept += keep ? 1U : 0U;
-                sum += keep ? dv : 0.0; // a sum is never -0, so +0 leaves it as it is
-            }
-        });
+        double sum = 0.0, ss = 0.0;
+        if (feeder)
+            R::template feed<G>(ring);
+        else
+            sum = clipped_sum<false>(rows, centre, cut, 0.0, kept);
         const double count = static_cast<double>(kept);
         if (live && count < 2.0)
             live = false;
         const double shift = live ? sum / count : 0.0;
-        if (!__any_sync(0xFFFFFFFFU, live))
+        if (!__syncthreads_or(live))
             break;
-        double ss = 0.0;
-        sweep([&](auto nb, const float* x) {
-#pragma unroll
-            for (int j = 0; j < nb; ++j) {
-                const double dv = x[j] - centre;
-                ss += fabs(dv) <= cut ? (dv - shift) * (dv - shift) : 0.0;
-            }
-        });
+        if (feeder) {
+            R::template feed<G>(ring);
+        } else {
+            uint32_t ignored;
+            ss = clipped_sum<true>(rows, centre, cut, shift, ignored);
+        }
         if (live) {
             const double clipped = sqrt(ss / count);
             if (!(clipped > 0.0)) {
@@ -445,117 +491,186 @@ __global__ void __launch_bounds__(32)
 
 // ---- moments --------------------------------------------------------------
 
-// One (window, channel) sequence of the moments pass, fed in time order
-// (lib/cpu/rfi_cpu_measure.cpp:91-138).
-struct MomentsAcc {
-    MomentSums s{0, 0, 0, 0, 0, 0, 0, 0, 0};
-    uint32_t n = 0, nc = 0; // the counts s.n and s.nc, kept as integers (exact)
-    double prev = 0.0;
-    float l, iv;
-    double clip;
-    uint64_t b;
-    __device__ __forceinline__ void step(float x, uint64_t t) {
-        const double z  = (x - l) * iv;
-        const double z2 = z * z;
-        ++n;
-        s.s1 += z;
-        s.s2 += z2;
-        s.s3 += z2 * z;
-        s.s4 += z2 * z2;
-        if (t > b)
-            s.lag += z * prev;
-        prev = z;
-        if (fabs(z) <= clip) {
-            ++nc;
-            s.c1 += z;
-            s.c2 += z2;
-        }
-    }
-    __device__ __forceinline__ MomentSums sums() const {
-        MomentSums r = s;
-        r.n          = static_cast<double>(n);
-        r.nc         = static_cast<double>(nc);
-        return r;
-    }
-};
+// The moments of a window's channels in time order
+// (lib/cpu/rfi_cpu_measure.cpp:91-138): nine running sums of z, its powers,
+// its product with the previous z and the clipped sums, a lane per channel
+// and 32 channels a CTA, streamed as rfi_columns.cuh says. Every sum is its
+// own chain of FP64 additions, so ROLES warps of a CTA can keep them apart,
+// each reading the same columns: with ROLES = 3 (where groups are few) a
+// warp carries two or three sums (z and z^2 are formed again in each), with
+// 1 all of them. 1024 float32 channels, 2 windows of 31 250 rows: 430 us
+// (1611 with one warp's sums behind block-wide stages); 4096 uint8 channels,
+// 8 windows: 1410 us (1976), where 12 FP64 operations a sample bound it.
 
-template <int D>
-__global__ void k_moments(Dims d, const uint8_t* __restrict__ raw, const float* __restrict__ loc,
-                          const float* __restrict__ inv, const uint8_t* __restrict__ static_mask,
-                          float clip, MomentSums* __restrict__ out) {
-    const uint64_t c = blockIdx.x * static_cast<uint64_t>(blockDim.x) + threadIdx.x;
-    const uint64_t w = blockIdx.y;
-    if (c >= d.nchans)
-        return;
-    const uint64_t o = w * d.nchans + c;
-    const uint64_t b = window_begin(w, d.window), e = window_end(w, d);
-    MomentsAcc acc;
-    acc.l    = loc[o];
-    acc.iv   = inv[o];
-    acc.clip = clip;
-    acc.b    = b;
-    if (static_mask[c] != 0 && acc.iv != 0.0F) {
-        // Rows are fetched kBlock at a time (independent loads in flight),
-        // then consumed strictly in time order.
-        for (uint64_t t0 = b; t0 < e; t0 += kBlock) {
-            float xs[kBlock];
+template <int ROLES, int ROLE, class R, class Z>
+__device__ __forceinline__ void moments_walk(const R& rows, Z&& z_of, float clip, MomentSums& out) {
+    constexpr bool kLow  = ROLES == 1 || ROLE == 0; // s1, s2, lag
+    constexpr bool kHigh = ROLES == 1 || ROLE == 1; // s3, s4
+    constexpr bool kClip = ROLES == 1 || ROLE == 2; // nc, c1, c2
+    constexpr int A      = cols::kAhead;
+    double s1 = 0.0, s2 = 0.0, s3 = 0.0, s4 = 0.0, lag = 0.0, c1 = 0.0, c2 = 0.0;
+    uint32_t nc = 0;
+    uint32_t raw[A];
+    double z[4];                // widened 3 rows ahead
+    double z2[2], z3[2], lp[2]; // z^2, z^3 and the lag product a row ahead
+    const double wide_clip = clip;
+    // the products of row j (z of row j - 1 given) into slot k
+    auto products = [&](int k, double zj, double before, bool first) {
+        cols::mul(z2[k], zj, zj);
+        if constexpr (kLow) {
+            cols::mul(lp[k], zj, before);
+            if (first)
+                lp[k] = 0.0;
+        }
+        if constexpr (kHigh)
+            cols::mul(z3[k], z2[k], zj);
+    };
+    auto sums = [&](double zj, double q2, double q3, double l) {
+        if constexpr (kLow) {
+            cols::add(s1, s1, zj);
+            cols::add(s2, s2, q2);
+            cols::add(lag, lag, l);
+        }
+        if constexpr (kHigh) {
+            double q4;
+            cols::mul(q4, q2, q2);
+            cols::add(s3, s3, q3);
+            cols::add(s4, s4, q4);
+        }
+        if constexpr (kClip) {
+            // sums from +0 are never -0, so adding +0 leaves them as they are
+            double k1, k2;
+            uint32_t one;
+            cols::keep(k1, one, zj, wide_clip);
+            k2 = one != 0 ? q2 : 0.0;
+            nc += one;
+            cols::add(c1, c1, k1);
+            cols::add(c2, c2, k2);
+        }
+    };
+    double tail_prev = 0.0;
+    rows.walk(
+        [&](uint32_t a) {
 #pragma unroll
-            for (int j = 0; j < kBlock; ++j)
-                xs[j] = t0 + j < e ? rd<D>(raw + (t0 + j) * d.row_bytes, c) : 0.0F;
+            for (int j = 0; j < A; ++j)
+                raw[j] = rows.bits(a + j * R::kPitch, j);
 #pragma unroll
-            for (int j = 0; j < kBlock; ++j) {
-                if (t0 + j >= e)
-                    break;
-                acc.step(xs[j], t0 + j);
+            for (int j = 0; j < 3; ++j)
+                cols::widen(z[j], z_of(raw[j]));
+            products(0, z[0], 0.0, true);
+        },
+        [&](int r, uint32_t a, uint32_t b) {
+#pragma unroll
+            for (int j = 0; j < cols::kBatch; ++j) {
+                const float ahead = z_of(raw[(j + 3) % A]);
+                raw[j % A] = rows.bits(j + A < cols::kBatch ? a + (j + A) * R::kPitch
+                                                            : b + (j + A - cols::kBatch) * R::kPitch, r + j + A);
+                products((j + 1) & 1, z[(j + 1) & 3], z[j & 3], false);
+                cols::widen(z[(j + 3) & 3], ahead);
+                sums(z[j & 3], z2[j & 1], z3[j & 1], lp[j & 1]);
             }
-        }
+            tail_prev = z[(cols::kBatch - 1) & 3];
+        },
+        [&](int r, uint32_t a) {
+            double zj;
+            cols::widen(zj, z_of(rows.bits(a, r)));
+            products(0, zj, tail_prev, r == 0);
+            sums(zj, z2[0], z3[0], lp[0]);
+            tail_prev = zj;
+        });
+    if constexpr (kLow) {
+        out.s1  = s1;
+        out.s2  = s2;
+        out.lag = lag;
     }
-    out[o] = acc.sums();
+    if constexpr (kHigh) {
+        out.s3 = s3;
+        out.s4 = s4;
+    }
+    if constexpr (kClip) {
+        out.nc = static_cast<double>(nc);
+        out.c1 = c1;
+        out.c2 = c2;
+    }
 }
 
-// The same sequences with the block's channel columns streamed through
-// shared memory (rfi_stage.cuh): one thread per channel of a
-// kStageChans-channel segment.
-constexpr int kStageChans = 128;
+template <int D, int U, int G>
+using MomentRing = cols::Ring<static_cast<int>(kBitsOf<D>), U, kBitsOf<D> < 32 ? 128 : G == 1 ? 64 : 32, 4>;
 
-template <int D>
-__global__ void __launch_bounds__(kStageChans)
-    k_moments_staged(Dims d, const uint8_t* __restrict__ raw, const float* __restrict__ loc,
-                     const float* __restrict__ inv, const uint8_t* __restrict__ static_mask,
-                     float clip, MomentSums* __restrict__ out, int seg_bytes, int rows) {
-    extern __shared__ __align__(16) uint8_t stage_buf[];
-    const uint64_t c0 = static_cast<uint64_t>(blockIdx.x) * kStageChans;
-    const uint64_t c  = c0 + threadIdx.x;
-    const uint64_t w  = blockIdx.y;
-    const bool in     = c < d.nchans;
-    const uint64_t o  = w * d.nchans + c;
+// The float of a sample's stored bits (codes of 16 bits or less by the
+// exponent of 2^23 and one subtraction: the conversion unit is left to the
+// widening).
+template <int D> __device__ __forceinline__ float sample_of(uint32_t v) {
+    if constexpr (D == FROST_FLOAT32)
+        return __uint_as_float(v);
+    else if constexpr (D == FROST_UINT32)
+        return static_cast<float>(v);
+    else
+        return __uint_as_float(0x4B000000U | v) - 8388608.0F;
+}
+
+template <int D, int U, int G>
+__global__ void __launch_bounds__(G == 1 ? 128 : 32 * (G + 1))
+    k_moments(Dims d, const uint8_t* __restrict__ raw, const float* __restrict__ loc, const float* __restrict__ inv,
+              const uint8_t* __restrict__ static_mask, float clip, MomentSums* __restrict__ out) {
+    using R = MomentRing<D, U, G>;
+    constexpr int kRoles = G == 1 ? 3 : 1;
+    extern __shared__ __align__(16) uint8_t rings[]; // [G][R::kBytes]
+    const int warp       = static_cast<int>(threadIdx.x >> 5U);
+    const uint64_t first = static_cast<uint64_t>(blockIdx.x) * 32 * G;
+    const uint64_t w     = blockIdx.y;
     const uint64_t b = window_begin(w, d.window), e = window_end(w, d);
-    MomentsAcc acc;
-    acc.l    = in ? loc[o] : 0.0F;
-    acc.iv   = in ? inv[o] : 0.0F;
-    acc.clip = clip;
-    acc.b    = b;
-    const bool active   = in && static_mask[c] != 0 && acc.iv != 0.0F;
-    const uint64_t off  = c0 * kBitsOf<D> / 8;
-    const uint64_t left = d.row_bytes - off;
-    const int copy      = static_cast<int>(left < static_cast<uint64_t>(seg_bytes) ? left : seg_bytes);
-    stage::StagerN<kDeepStages> st(stage_buf, raw + off, d.row_bytes, seg_bytes, copy, rows, b, e);
-    st.start();
-    for (int k = 0; k < st.nblk; ++k) {
-        st.wait(k);
-        const uint8_t* buf = st.buf(k);
-        const int nr       = st.rows_of(k);
-        const uint64_t t0  = st.t0(k);
-        if (active) {
-#pragma unroll 8
-            for (int r = 0; r < nr; ++r)
-                acc.step(rd<D>(buf + r * seg_bytes, threadIdx.x), t0 + r);
+    auto ring = [&](int g) {
+        const uint64_t c0 = first + 32 * static_cast<uint64_t>(g), off = c0 * kBitsOf<D> / 8;
+        return R(rings + g * R::kBytes, raw + b * d.row_bytes + off, d.row_bytes,
+                 c0 < d.nchans ? d.row_bytes - off : 0, e - b);
+    };
+    const int group   = warp == 0 || G == 1 ? 0 : warp - 1;
+    const uint64_t c  = first + 32 * static_cast<uint64_t>(group) + (threadIdx.x & 31U);
+    const bool in     = warp != 0 && c < d.nchans;
+    const uint64_t o  = w * d.nchans + c;
+    const float l     = in ? loc[o] : 0.0F;
+    const float iv    = in ? inv[o] : 0.0F;
+    const bool active = in && static_mask[c] != 0 && iv != 0.0F;
+    MomentSums s{0, 0, 0, 0, 0, 0, 0, 0, 0};
+    if (__syncthreads_or(active)) {
+        if (warp == 0) {
+            R::template feed<G>(ring);
+            return;
         }
-        st.release(k);
+        const R rows = ring(group);
+        auto z_of    = [&](uint32_t v) { return (sample_of<D>(v) - l) * iv; };
+        if (kRoles == 1 || warp == 1)
+            moments_walk<kRoles, 0>(rows, z_of, clip, s);
+        else if (warp == 2)
+            moments_walk<kRoles, 1>(rows, z_of, clip, s);
+        else
+            moments_walk<kRoles, 2>(rows, z_of, clip, s);
+        if (!active)
+            s = MomentSums{0, 0, 0, 0, 0, 0, 0, 0, 0};
     }
-    if (in)
-        out[o] = acc.sums();
+    if (!in)
+        return;
+    MomentSums& to = out[o];
+    if (kRoles == 1 || warp == 1) {
+        to.n   = active ? static_cast<double>(e - b) : 0.0;
+        to.s1  = s.s1;
+        to.s2  = s.s2;
+        to.lag = s.lag;
+    }
+    if (kRoles == 1 || warp == 2) {
+        to.s3 = s.s3;
+        to.s4 = s.s4;
+    }
+    if (kRoles == 1 || warp == 3) {
+        to.nc = s.nc;
+        to.c1 = s.c1;
+        to.c2 = s.c2;
+    }
 }
+
+// Channels of a staged segment of the column scan (rfi_stage.cuh).
+constexpr int kStageChans = 128;
 
 // ---- row scan ---------------------------------------------------------------
 
@@ -1432,150 +1547,103 @@ __global__ void k_unpack(Dims d, const uint8_t* __restrict__ raw, float* __restr
 // lies at least 2^-54 / n relative from every midpoint, far more than
 // 2^-104 for n < 2^40, so q is the correctly rounded quotient, as
 // Markstein-style corrections argue (P. Markstein, IBM J. Res. Develop. 34,
-// 1990; Muller et al., Handbook of Floating-Point Arithmetic, ch. 4). Tiny
-// nonzero |delta| (where delta * y_lo could lose bits) takes the plain
-// division. The plain division as a call, so the compiler keeps it off the
-// common path instead of computing it alongside (if-converting the branch).
-__device__ __noinline__ double div_plain(double a, double n) { return a / n; }
+// 1990; Muller et al., Handbook of Floating-Point Arithmetic, ch. 4).
+//
+// A nonzero delta is never so small that delta * y_lo loses bits, so the
+// form needs no branch. Samples are floats: zero or at least 2^-149. Let m
+// be the mean before a row n < 2^31. A row x != 0 leaves |mean| >= 2^-236
+// or 0: with |m| <= 2^-183, |q| >= 2^-182 outweighs m; else m is a multiple
+// of 2^-235, and q is either below 2^-184 or a multiple of 2^-236. Rows of
+// zeros scale the mean by the product of (1 - 1/n), at least 2^-32 in all.
+// So a nonzero mean stays above 2^-268 and is a multiple of 2^-320, as is
+// x - mean: delta * y_lo is a normal number.
 
-// One (window, channel) Welford sequence of the re-measure after a
-// transform (lib/cpu/rfi_cpu.cpp:219-238). The mean never becomes -0 (it
-// starts at +0 and a rounded sum is -0 only when both terms are), so a zero
-// quotient (delta = +-0) leaves it unchanged without a select.
-struct WelfordAcc {
-    double mean = 0.0, var = 0.0;
-    uint64_t b;
-    const double* recip; // recip[2n], recip[2n + 1] = y_hi, y_lo of 1/n, or null for the plain division
-    __device__ __forceinline__ void step(float xf, uint64_t t) {
-        const uint64_t n = t - b + 1;
-        if (recip != nullptr)
-            step_recip(xf, static_cast<double>(n), recip[2 * n], recip[2 * n + 1]);
-        else
-            step_plain(xf, static_cast<double>(n));
-    }
-    __device__ __forceinline__ void step_plain(float xf, double n) {
-        const double x     = xf;
-        const double delta = x - mean;
-        mean += div_plain(delta, n);
-        var += delta * (x - mean);
-    }
-    /** step_recip without the tiny-numerator branch: `bad` records that
-     * the step needed it (the caller then redoes the steps with it). */
-    __device__ __forceinline__ void step_fast(float xf, double yh, double yl, bool& bad) {
-        const double x     = xf;
-        const double delta = x - mean;
-        bad |= !(fabs(delta) > 0x1p-900) && delta != 0.0;
-        mean += fma(delta, yh, delta * yl);
-        var += delta * (x - mean);
-    }
-    /** The update for the n-th sample given the two-term reciprocal of n. */
-    __device__ __forceinline__ void step_recip(float xf, double n, double yh, double yl) {
-        const double x     = xf;
-        const double delta = x - mean;
-        double q           = fma(delta, yh, delta * yl);
-        if (!(fabs(delta) > 0x1p-900) && delta != 0.0)
-            q = div_plain(delta, n);
-        mean += q;
-        var += delta * (x - mean);
-    }
-};
+// The Welford statistics of the re-measure after a transform
+// (lib/cpu/rfi_cpu.cpp:219-238): a lane per channel, a CTA per 32 channels
+// of a window; a row's samples and its count's two-term reciprocal are
+// streamed together (rfi_columns.cuh). Bound by the chain of four dependent
+// FP64 operations a row (32 cycles) where groups are few, by issue where
+// they are many. The mean never becomes -0 (it starts at +0 and a rounded
+// sum is -0 only when both terms are), so a zero quotient (delta = +-0)
+// leaves it unchanged without a select. var's increment is added a row late,
+// in the chain's gaps. 1024 channels, 2 windows of 31 250 rows: 690 us (2276
+// before: 126 cycles a row); 4096 channels, 8 windows: 1350 us (2979).
+template <int U, int G> using WorkRing = cols::Ring<32, U, G == 1 ? 64 : 32, 4, true>;
 
-__global__ void k_welford(Dims d, const float* __restrict__ work, const double* __restrict__ recip,
-                          float* __restrict__ loc, float* __restrict__ scale) {
-    const uint64_t c = blockIdx.x * static_cast<uint64_t>(blockDim.x) + threadIdx.x;
-    const uint64_t w = blockIdx.y;
-    if (c >= d.nchans)
-        return;
+template <int U, int G>
+__global__ void __launch_bounds__(32 * (G + 1))
+    k_welford(Dims d, const float* __restrict__ work, const double* __restrict__ recip, float* __restrict__ loc,
+              float* __restrict__ scale) {
+    using R = WorkRing<U, G>;
+    extern __shared__ __align__(16) uint8_t rings[]; // [G][R::kBytes], the records
+    const uint64_t first = static_cast<uint64_t>(blockIdx.x) * 32 * G;
+    const uint64_t w     = blockIdx.y;
+    const uint64_t n     = d.nchans;
     const uint64_t b = window_begin(w, d.window), e = window_end(w, d);
-    WelfordAcc acc{0.0, 0.0, b, recip};
-    for (uint64_t tb = b; tb < e; tb += kBlock) {
-        float xs[kBlock];
-#pragma unroll
-        for (int q = 0; q < kBlock; ++q)
-            xs[q] = tb + q < e ? work[(tb + q) * d.nchans + c] : 0.0F;
-#pragma unroll
-        for (int q = 0; q < kBlock; ++q) {
-            if (tb + q >= e)
-                break;
-            acc.step(xs[q], tb + q);
-        }
-    }
-    loc[w * d.nchans + c]   = static_cast<float>(acc.mean);
-    scale[w * d.nchans + c] = e > b ? static_cast<float>(sqrt(acc.var / static_cast<double>(e - b))) : 0.0F;
-}
-
-__global__ void __launch_bounds__(kStageChans)
-    k_welford_staged(Dims d, const float* __restrict__ work, const double* __restrict__ recip,
-                     float* __restrict__ loc, float* __restrict__ scale, int seg_bytes, int rows) {
-    extern __shared__ __align__(16) uint8_t stage_buf[];
-    __shared__ double2 ys[kDeepStages][kStageChans]; // two-term reciprocals of each stage's rows
-    const uint64_t c0 = static_cast<uint64_t>(blockIdx.x) * kStageChans;
-    const uint64_t c  = c0 + threadIdx.x;
-    const uint64_t w  = blockIdx.y;
-    const bool in     = c < d.nchans;
-    const uint64_t b = window_begin(w, d.window), e = window_end(w, d);
-    WelfordAcc acc{0.0, 0.0, b, recip};
-    const uint64_t pitch = d.nchans * sizeof(float);
-    const uint64_t left  = pitch - c0 * sizeof(float);
-    const int copy       = static_cast<int>(left < static_cast<uint64_t>(seg_bytes) ? left : seg_bytes);
-    const int stride     = seg_bytes / static_cast<int>(sizeof(float));
-    stage::StagerN<kDeepStages> st(stage_buf, reinterpret_cast<const uint8_t*>(work + c0), pitch, seg_bytes,
-                                   copy, rows, b, e);
-    // The reciprocals of a stage's counts are read into shared memory with
-    // the stage, so no load sits on the sequential update chain.
-    auto load_recip = [&](int k) {
-        if (k < st.nblk && static_cast<int>(threadIdx.x) < st.rows_of(k)) {
-            const uint64_t n = st.t0(k) - b + 1 + threadIdx.x;
-            ys[k % kDeepStages][threadIdx.x] = recip != nullptr ? make_double2(recip[2 * n], recip[2 * n + 1])
-                                                                : make_double2(0.0, 0.0);
-        }
+    auto ring = [&](int g) {
+        const uint64_t c0 = first + 32 * static_cast<uint64_t>(g);
+        // record r: the reciprocal of r + 1
+        return R(rings + g * R::kBytes, reinterpret_cast<const uint8_t*>(work + b * n + c0), n * sizeof(float),
+                 c0 < n ? (n - c0) * sizeof(float) : 0, e - b, rings + G * R::kBytes,
+                 g == 0 ? reinterpret_cast<const double2*>(recip) + 1 : nullptr);
     };
-    for (int k = 0; k < kDeepStages; ++k)
-        load_recip(k);
-    st.start();
-    for (int k = 0; k < st.nblk; ++k) {
-        st.wait(k);
-        const float* buf  = reinterpret_cast<const float*>(st.buf(k));
-        const int nr      = st.rows_of(k);
-        double nd         = static_cast<double>(st.t0(k) - b); // exact below 2^53
-        if (in) {
-            if (recip != nullptr) {
-                // Eight steps at a time without a branch on the update chain;
-                // the rare eight with a tiny nonzero numerator are redone with
-                // the plain division where it is needed.
-                const double2* yk = ys[k % kDeepStages];
-                for (int r0 = 0; r0 < nr; r0 += 8) {
-                    const double m0 = acc.mean, v0 = acc.var;
-                    bool bad        = false;
-                    if (r0 + 8 <= nr) {
-#pragma unroll
-                        for (int r = r0; r < r0 + 8; ++r)
-                            acc.step_fast(buf[r * stride + threadIdx.x], yk[r].x, yk[r].y, bad);
-                    } else {
-                        for (int r = r0; r < nr; ++r)
-                            acc.step_fast(buf[r * stride + threadIdx.x], yk[r].x, yk[r].y, bad);
-                    }
-                    if (bad) {
-                        acc.mean = m0;
-                        acc.var  = v0;
-                        for (int r = r0; r < min(r0 + 8, nr); ++r)
-                            acc.step_recip(buf[r * stride + threadIdx.x], nd + (r + 1), yk[r].x, yk[r].y);
-                    }
-                }
-            } else {
-                for (int r = 0; r < nr; ++r) {
-                    nd += 1.0;
-                    acc.step_plain(buf[r * stride + threadIdx.x], nd);
-                }
-            }
-        }
-        st.release(k);
-        load_recip(k + kDeepStages);
+    if (threadIdx.x < 32) {
+        R::template feed<G>(ring);
+        return;
     }
-    if (in) {
-        loc[w * d.nchans + c] = static_cast<float>(acc.mean);
-        scale[w * d.nchans + c] =
-            e > b ? static_cast<float>(sqrt(acc.var / static_cast<double>(e - b))) : 0.0F;
+    const uint64_t c = first + threadIdx.x - 32;
+    const R rows     = ring(static_cast<int>(threadIdx.x >> 5U) - 1);
+    constexpr int A = cols::kAhead;
+    double mean = 0.0, var = 0.0;
+    double pd = 0.0, pr = 0.0; // the last row's delta and x - mean
+    uint32_t raw[A];
+    double x[2], yh[4], yl[4]; // widened 2 rows ahead, reciprocals read 4
+    rows.walk(
+        [&](uint32_t a) {
+#pragma unroll
+            for (int j = 0; j < A; ++j)
+                raw[j] = rows.bits(a + j * R::kPitch, j);
+#pragma unroll
+            for (int j = 0; j < 4; ++j)
+                cols::pair(yh[j], yl[j], rows.record(j));
+            cols::widen(x[0], __uint_as_float(raw[0]));
+            cols::widen(x[1], __uint_as_float(raw[1]));
+        },
+        [&](int r, uint32_t a, uint32_t after) {
+            const uint32_t ya = rows.record(r), yb = rows.record(r + cols::kBatch);
+#pragma unroll
+            for (int j = 0; j < cols::kBatch; ++j) {
+                double delta, u, q, pv;
+                const double xj = x[j & 1];
+                cols::sub(delta, xj, mean);
+                raw[j % A] = rows.bits(j + A < cols::kBatch ? a + (j + A) * R::kPitch
+                                                            : after + (j + A - cols::kBatch) * R::kPitch, r + j + A);
+                cols::mul(pv, pd, pr);
+                cols::mul(u, delta, yl[j & 3]);
+                cols::widen(x[j & 1], __uint_as_float(raw[(j + 2) % A]));
+                cols::add(var, var, pv);
+                cols::fma(q, delta, yh[j & 3], u);
+                cols::pair(yh[j & 3], yl[j & 3], j + 4 < cols::kBatch ? ya + (j + 4) * 16
+                                                                      : yb + (j + 4 - cols::kBatch) * 16);
+                pd = delta;
+                cols::add(mean, mean, q);
+                cols::sub(pr, xj, mean);
+            }
+        },
+        [&](int r, uint32_t a) {
+            var += pd * pr;
+            const double xj    = __uint_as_float(rows.bits(a, r));
+            const double delta = xj - mean;
+            double h, l;
+            cols::pair(h, l, rows.record(r));
+            mean += ::fma(delta, h, delta * l);
+            pd = delta;
+            pr = xj - mean;
+        });
+    var += pd * pr;
+    if (c < d.nchans) {
+        loc[w * d.nchans + c]   = static_cast<float>(mean);
+        scale[w * d.nchans + c] = e > b ? static_cast<float>(sqrt(var / static_cast<double>(e - b))) : 0.0F;
     }
 }
 
@@ -1765,6 +1833,21 @@ static void set_smem(const void* fn, size_t bytes) {
         allow_large_smem(fn);
 }
 
+// f(copy bytes, groups a CTA) for a column kernel of `groups` 32-channel groups.
+template <int WIDE = 16, class F> static void on_groups(uint64_t groups, bool aligned, F&& f) {
+    using One  = std::integral_constant<int, 1>;
+    using Many = std::integral_constant<int, cols::kManyGroups>;
+    const bool few = cols::few_groups(groups);
+    if (aligned && few)
+        f(std::integral_constant<int, WIDE>{}, One{});
+    else if (aligned)
+        f(std::integral_constant<int, WIDE>{}, Many{});
+    else if (few)
+        f(std::integral_constant<int, 4>{}, One{});
+    else
+        f(std::integral_constant<int, 4>{}, Many{});
+}
+
 void launch_check_finite(const uint8_t* raw, uint64_t nwords, unsigned long long* first_bad,
                          cudaStream_t s) {
     if (nwords == 0)
@@ -1788,10 +1871,15 @@ void launch_bandpass(const Dims& d, const float* samples, float* loc, float* sca
     FB_COUNT_LAUNCH();
     k_remedian<true><<<grid, 32 * kRemedianWarps, 0, s>>>(d, samples, loc, scale, inv);
     FB_COUNT_LAUNCH();
-    if (d.nchans % 4 == 0 && reinterpret_cast<uintptr_t>(samples) % 16 == 0)
-        k_bandpass_refine<16><<<grid, 32, 0, s>>>(d, samples, loc, scale, inv, unmeasured);
-    else
-        k_bandpass_refine<4><<<grid, 32, 0, s>>>(d, samples, loc, scale, inv, unmeasured);
+    auto refine = [&](auto u, auto groups) {
+        constexpr int U = decltype(u)::value, G = decltype(groups)::value;
+        constexpr size_t smem = G * SampleRing<U, G>::kBytes;
+        set_smem(reinterpret_cast<const void*>(&k_bandpass_refine<U, G>), smem);
+        const dim3 g(grid1(d.nchans, 32 * G), static_cast<unsigned>(d.nwin));
+        k_bandpass_refine<U, G><<<g, 32 * (G + 1), smem, s>>>(d, samples, loc, scale, inv, unmeasured);
+    };
+    on_groups(static_cast<uint64_t>(grid.x) * grid.y,
+              d.nchans % 4 == 0 && reinterpret_cast<uintptr_t>(samples) % 16 == 0, refine);
     FB_COUNT_LAUNCH();
 }
 
@@ -1803,7 +1891,6 @@ constexpr int kStageBytes = 16 * 1024;
 struct StageGeom {
     int seg_bytes = 0, rows = 0;
     size_t smem() const { return 2 * static_cast<size_t>(seg_bytes) * rows; }
-    size_t smem_deep() const { return kDeepStages * static_cast<size_t>(seg_bytes) * rows; }
 };
 
 bool aligned16(const void* p) { return reinterpret_cast<uintptr_t>(p) % 16 == 0; }
@@ -1821,18 +1908,18 @@ StageGeom stage_geom(const void* base, uint64_t row_bytes, int bits) {
 
 void launch_moments(const Dims& d, const uint8_t* raw, const float* loc, const float* inv,
                     const uint8_t* static_mask, float clip, MomentSums* out, cudaStream_t s) {
-    const StageGeom g = stage_geom(raw, d.row_bytes, bits_of(d.dtype));
-    if (g.seg_bytes == 0) {
-        const dim3 grid(grid1(d.nchans, 64), static_cast<unsigned>(d.nwin));
-        FB_DISPATCH(d.dtype, k_moments<D><<<grid, 64, 0, s>>>(d, raw, loc, inv, static_mask, clip, out));
-    } else {
-        const dim3 grid(grid1(d.nchans, kStageChans), static_cast<unsigned>(d.nwin));
-        FB_DISPATCH(d.dtype, {
-            set_smem(reinterpret_cast<const void*>(&k_moments_staged<D>), g.smem_deep());
-            k_moments_staged<D><<<grid, kStageChans, g.smem_deep(), s>>>(d, raw, loc, inv, static_mask, clip, out,
-                                                                        g.seg_bytes, g.rows);
-        });
-    }
+    FB_DISPATCH(d.dtype, {
+        constexpr int kWide = kBitsOf<D> >= 4 ? 16 : 4; // 32 narrower samples are no 16 bytes
+        on_groups<kWide>(grid1(d.nchans, 32) * d.nwin, aligned16(raw) && d.row_bytes % 16 == 0,
+                         [&](auto u, auto groups) {
+                             constexpr int U = decltype(u)::value, G = decltype(groups)::value;
+                             constexpr size_t smem = G * MomentRing<D, U, G>::kBytes;
+                             set_smem(reinterpret_cast<const void*>(&k_moments<D, U, G>), smem);
+                             const dim3 g(grid1(d.nchans, 32 * G), static_cast<unsigned>(d.nwin));
+                             k_moments<D, U, G><<<g, G == 1 ? 128 : 32 * (G + 1), smem, s>>>(
+                                 d, raw, loc, inv, static_mask, clip, out);
+                         });
+    });
     FB_COUNT_LAUNCH();
 }
 
@@ -1990,18 +2077,13 @@ void launch_unpack(const Dims& d, const uint8_t* raw, float* work, cudaStream_t 
 
 void launch_welford(const Dims& d, const float* work, const double* recip, float* loc, float* scale,
                     cudaStream_t s) {
-    const StageGeom g = stage_geom(work, d.nchans * sizeof(float), 32);
-    if (g.seg_bytes == 0) {
-        const dim3 grid(grid1(d.nchans, 64), static_cast<unsigned>(d.nwin));
-        k_welford<<<grid, 64, 0, s>>>(d, work, recip, loc, scale);
-    } else {
-        const dim3 grid(grid1(d.nchans, kStageChans), static_cast<unsigned>(d.nwin));
-        // a stage's reciprocals are loaded one per thread
-        const int rows    = std::min(g.rows, kStageChans);
-        const size_t smem = kDeepStages * static_cast<size_t>(g.seg_bytes) * rows;
-        set_smem(reinterpret_cast<const void*>(&k_welford_staged), smem);
-        k_welford_staged<<<grid, kStageChans, smem, s>>>(d, work, recip, loc, scale, g.seg_bytes, rows);
-    }
+    on_groups(grid1(d.nchans, 32) * d.nwin, aligned16(work) && d.nchans % 4 == 0, [&](auto u, auto groups) {
+        constexpr int U = decltype(u)::value, G = decltype(groups)::value;
+        constexpr size_t smem = G * WorkRing<U, G>::kBytes + WorkRing<U, G>::kSideBytes;
+        set_smem(reinterpret_cast<const void*>(&k_welford<U, G>), smem);
+        const dim3 g(grid1(d.nchans, 32 * G), static_cast<unsigned>(d.nwin));
+        k_welford<U, G><<<g, 32 * (G + 1), smem, s>>>(d, work, recip, loc, scale);
+    });
     FB_COUNT_LAUNCH();
 }
 

@@ -5,11 +5,14 @@ against the same arithmetic in numpy: sums in row order (np.cumsum), every
 operation rounded as the reference's strict IEEE build rounds it. The bar is
 bit equality."""
 
+import json
+
 import numpy as np
 import pytest
 
-from frost_b200.config import BlockLayout, DataType, RfiConfig
-from tests.rfi_cases import pack
+from frost_b200.config import BlockLayout, DataType, RfiConfig, ZeroDMMode
+from tests.rfi_cases import CASES, make_case, pack
+from tests.test_rfi_gpu import GOLDEN, digest
 
 MAX_ROWS = 3125
 
@@ -52,7 +55,14 @@ def bandpass(x):
         clipped = np.sqrt(ss / np.maximum(count, 1))
         live &= clipped > 0
         centre, sd = np.where(live, centre + shift, centre), np.where(live, clipped, sd)
-    return centre.astype(np.float32), sd.astype(np.float32)
+    return centre.astype(np.float32), np.where(v.min(0) < v.max(0), sd, 0).astype(np.float32)
+
+
+def same_measured(got, want, scales):
+    """Bit equality of every cell of a measured (window, channel): one whose
+    sampled values are all equal has no scale, and its cells are filled."""
+    on = np.concatenate([np.repeat(s[:, None] > 0, e - b, axis=1) for (b, e), s in scales], axis=1)
+    return np.array_equal(got.view(np.uint32)[on], want.view(np.uint32)[on])
 
 
 def samples(rng, nsamps, nchans, dtype):
@@ -71,15 +81,85 @@ def samples(rng, nsamps, nchans, dtype):
 @pytest.mark.parametrize("nchans,nsamps,window,dtype", [
     (1, 64, 64, DataType.FLOAT32), (31, 127, 127, DataType.UINT8), (33, 640, 130, DataType.FLOAT32),
     (64, 4096, 2000, DataType.UINT8), (100, 9001, 4000, DataType.UINT16), (104, 3300, 3200, DataType.UINT2),
-    (161, 6400, 3125, DataType.FLOAT32)])
+    (161, 6400, 3125, DataType.FLOAT32), (1001, 1300, 130, DataType.UINT8), (1024, 1000, 100, DataType.FLOAT32)])
 def test_bandpass_levels_and_scales(nchans, nsamps, window, dtype):
     from frost_b200.rfi import RFICleaner
     rng = np.random.default_rng(nchans * 7919 + nsamps)
     x = samples(rng, nsamps, nchans, dtype)
     gpu = RFICleaner(RfiConfig.quiet(), BlockLayout(nchans, nsamps, dtype, 2.0 ** -10, 1400.0, 1.0), window * 2.0 ** -10)
     got = gpu.execute_normalized(pack(x, dtype))
-    want = np.zeros((nchans, nsamps), np.float32)
+    want, scales = np.zeros((nchans, nsamps), np.float32), []
     for b, e in windows(nsamps, window):
         level, scale = bandpass(x[b:e])
-        want[:, b:e] = ((x[b:e] - level) * (np.float32(1) / scale)).T
-    assert np.array_equal(got.view(np.uint32), want.view(np.uint32))
+        scales.append(((b, e), scale))
+        with np.errstate(divide="ignore", invalid="ignore"):
+            want[:, b:e] = ((x[b:e] - level) * (np.float32(1) / scale)).T
+    assert same_measured(got, want, scales)
+
+
+def welford(x):
+    """(mean, std) float32 of each column of x, updated row by row in double."""
+    mean, var = np.zeros(x.shape[1]), np.zeros(x.shape[1])
+    for n, row in enumerate(x.astype(np.float64), 1):
+        delta = row - mean
+        mean = mean + delta / n
+        var = var + delta * (row - mean)
+    return mean.astype(np.float32), np.sqrt(var / x.shape[0]).astype(np.float32)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("nchans,nsamps,window", [(1, 64, 64), (33, 131, 65), (50, 2100, 1000), (128, 1041, 513),
+                                                  (1001, 1300, 130), (1024, 1000, 100)])
+def test_welford_remeasure(nchans, nsamps, window):
+    """equalize rescales the cleaned cells (0 + 1 * z for float32 input) and
+    calibrates them again by their Welford mean and std."""
+    from frost_b200.rfi import RFICleaner
+    rng = np.random.default_rng(nchans * 131 + nsamps)
+    x = samples(rng, nsamps, nchans, DataType.FLOAT32)
+    cfg = RfiConfig.quiet()
+    cfg.equalize = True
+    gpu = RFICleaner(cfg, BlockLayout(nchans, nsamps, DataType.FLOAT32, 2.0 ** -10, 1400.0, 1.0), window * 2.0 ** -10)
+    got = gpu.execute_normalized(pack(x, DataType.FLOAT32))
+    want, scales = np.zeros((nchans, nsamps), np.float32), []
+    for b, e in windows(nsamps, window):
+        level, scale = bandpass(x[b:e])
+        scales.append(((b, e), scale))
+        with np.errstate(divide="ignore", invalid="ignore"):
+            y = np.float32(0) + np.float32(1) * ((x[b:e] - level) * (np.float32(1) / scale))
+            mean, std = welford(y)
+            want[:, b:e] = ((y - mean) * (np.float32(1) / std)).T
+    assert same_measured(got, want, scales)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("nchans,nsamps,window", [(9, 200, 100), (41, 2100, 700), (130, 5000, 2500), (1001, 1300, 130),
+                                                  (1024, 1000, 100)])
+def test_moments_do_not_depend_on_the_sample_type(nchans, nsamps, window):
+    """The same values as uint8, uint16 and float32 (other copies, shifts and
+    conversions of the moments pass) give the same masks and output."""
+    from frost_b200.rfi import RFICleaner
+    rng = np.random.default_rng(nchans + nsamps)
+    x = samples(rng, nsamps, nchans, DataType.UINT8)
+    x[:, nchans // 2] = np.clip(np.rint(rng.normal(120, 40, nsamps)), 0, 255)
+    cfg = RfiConfig()
+    cfg.moments.enabled = cfg.iqrm.enabled = cfg.kadane_channel.enabled = True
+    cfg.zero_dm = ZeroDMMode.SUBTRACT
+    out = []
+    for dtype in (DataType.UINT8, DataType.UINT16, DataType.FLOAT32):
+        gpu = RFICleaner(cfg, BlockLayout(nchans, nsamps, dtype, 2.0 ** -10, 1400.0, 1.0), window * 2.0 ** -10)
+        out.append((digest(gpu.execute_normalized(pack(x, dtype))), digest(gpu.channel_mask()),
+                    gpu.report()["chans_moments"]))
+    assert out[0] == out[1] == out[2]
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("name", CASES)
+def test_golden_digests(name):
+    """The reference cleaner's committed digests of every strategy mix."""
+    from frost_b200.rfi import RFICleaner
+    golden = json.load(open(GOLDEN))[name]
+    cfg, layout, baseline, blocks = make_case(name)
+    gpu = RFICleaner(cfg, layout, baseline)
+    for step, (block, nsamps) in enumerate(blocks):
+        assert digest(gpu.execute_normalized(block, nsamps)) == golden[step]["out_sha256"]
+        assert digest(gpu.channel_mask()) == golden[step]["mask_sha256"]
