@@ -136,7 +136,10 @@ struct RowConst {
     int E[kMaxWidths];      // trapezoid half-weight edge, 0 for a boxcar
     float inv[kMaxWidths];  // 1/sigma
     float inv_or[kMaxWidths];
-    float thr[kMaxWidths];  // window-sum threshold thresh * sigma
+    // window-sum thresholds: thresh * sigma in steady chunks; elsewhere one
+    // that no window sum whose S/N exceeds thresh, by either variance, stays
+    // below
+    float thr[2][kMaxWidths];
 };
 
 // Window sum of width W (trapezoid edge E, 0 for a boxcar) ending at chunk
@@ -247,24 +250,13 @@ struct Seg {
     float best;
 };
 
-// S/N of set bit k for width wi, or the best over widths (first maximum)
-// for wi < 0.
+// S/N of chunk sample k at width wi: snr_general, whose checks all pass in a
+// steady chunk.
 __device__ __forceinline__ float bit_snr(const SearchParams& p, const RowConst& rc, const float* Q, int64_t c0,
-                                         int k, int wi, int32_t delay, int& bw) {
-    if (wi >= 0) {
-        bw = wi;
-        return snr_general(p, rc, Q, c0, k, wi, delay);
-    }
-    float best = FB_NEG_INF;
-    bw         = 0;
-    for (int w = 0; w < p.nwidths; ++w) {
-        const float s = snr_general(p, rc, Q, c0, k, w, delay);
-        if (s > best) {
-            best = s;
-            bw   = w;
-        }
-    }
-    return best;
+                                         int k, int wi, int32_t delay, bool steady) {
+    if (steady)
+        return wsum(Q, k, rc.W[wi], rc.E[wi]) * rc.inv[wi];
+    return snr_general(p, rc, Q, c0, k, wi, delay);
 }
 
 __device__ __forceinline__ RunState run_of(const RowConst& rc, int64_t c0, const Seg& g) {
@@ -288,8 +280,8 @@ __device__ __forceinline__ Seg shfl_seg(const Seg& g, int src) {
     return r;
 }
 
-// The runs of one chunk's mask for one width (or across widths, wi < 0), by
-// a whole warp: lane L takes the chunk's samples [L CH / 32, (L + 1) CH / 32)
+// The runs of one chunk's mask, by a whole warp (value(k, bw): the S/N of set
+// bit k and its width): lane L takes the chunk's samples [L CH / 32, (L + 1) CH / 32)
 // (cut at the last valid sample) and finds its maximal runs in time order
 // (S/N of each set bit, first maximum); runs that touch neither end of the
 // lane's share are complete and emitted at once. Lane 0 then joins, in time order, the runs that do
@@ -297,10 +289,10 @@ __device__ __forceinline__ Seg shfl_seg(const Seg& g, int src) {
 // previous chunk, exactly as a sequential walk over the bits would (the
 // strict comparison keeps the earliest maximum), emits the closed ones and
 // leaves `run` open when it reaches the chunk's last valid sample.
-template <int CH>
-__device__ __forceinline__ void walk_runs_warp(const SearchParams& p, const RowConst& rc, const float* Q, int64_t c0,
-                               int32_t delay, const uint32_t* bits, int wi, RunState& run,
-                               const SearchRow& row, uint32_t* count) {
+template <int CH, class V>
+__device__ __forceinline__ void walk_runs_warp(const SearchParams& p, const RowConst& rc, int64_t c0,
+                                               const uint32_t* bits, V&& value, RunState& run, const SearchRow& row,
+                                               uint32_t* count) {
     constexpr int kPerLane = CH / 32 / 32; // mask words per lane
     const int lane = threadIdx.x & 31;
     // the lane's share ends at its last sample or at the chunk's last valid one
@@ -325,7 +317,7 @@ __device__ __forceinline__ void walk_runs_warp(const SearchParams& p, const RowC
             const int k = (lane * kPerLane + wd) * 32 + __ffs(b) - 1;
             b &= b - 1;
             int bw;
-            const float sn = bit_snr(p, rc, Q, c0, k, wi, delay, bw);
+            const float sn = value(k, bw);
             if (open && k == prev + 1) {
                 if (sn > cur.best) {
                     cur.best   = sn;
@@ -407,6 +399,51 @@ __device__ __forceinline__ void walk_runs_warp(const SearchParams& p, const RowC
     }
 }
 
+// Every set sample's best S/N over the widths (first maximum), by the whole
+// CTA, into Q and (the width) `best_w`. One warp that evaluated every width
+// of its lanes' samples in turn took 1.1 ms of a 1.25 ms search of 67
+// channels with bright pulses; this leaves 0.3 ms. A call of its own, like
+// general_hits: their registers would be taken from the common path (7 % of
+// a noise chunk when inlined).
+template <int CH>
+__device__ __noinline__ void best_over_widths(const SearchParams& p, const RowConst& rc, float* Q, int64_t c0,
+                                              int32_t delay, bool steady, const uint32_t* any_bits, uint8_t* best_w) {
+    constexpr int P = CH / kThreads;
+    float best[P];
+    uint8_t bw[P];
+#pragma unroll
+    for (int j = 0; j < P; ++j) {
+        const int k = threadIdx.x + j * kThreads;
+        best[j]     = FB_NEG_INF;
+        bw[j]       = 0;
+        if ((any_bits[k >> 5] >> (k & 31)) & 1U)
+            for (int w = 0; w < p.nwidths; ++w) {
+                const float sn = bit_snr(p, rc, Q, c0, k, w, delay, steady);
+                if (sn > best[j]) {
+                    best[j] = sn;
+                    bw[j]   = static_cast<uint8_t>(w);
+                }
+            }
+    }
+    __syncthreads();
+#pragma unroll
+    for (int j = 0; j < P; ++j) {
+        Q[threadIdx.x + j * kThreads]      = best[j];
+        best_w[threadIdx.x + j * kThreads] = bw[j];
+    }
+    __syncthreads();
+}
+
+// Which of chunk samples k .. k + 3 exceed the threshold by the general S/N.
+__device__ __noinline__ uint32_t general_hits(const SearchParams& p, const RowConst& rc, const float* Q, int64_t c0,
+                                              int k, int wi, int32_t delay) {
+    uint32_t nib = 0U;
+#pragma unroll
+    for (int e = 0; e < 4; ++e)
+        nib |= snr_general(p, rc, Q, c0, k + e, wi, delay) > p.thresh ? 1U << e : 0U;
+    return nib;
+}
+
 // Words of the per-width bit masks [nw][chunk / 32].
 __host__ __device__ constexpr int search_bits_words(int nw, int chunk) { return nw * (chunk / 32); }
 
@@ -415,7 +452,7 @@ enum : int {
     kTestExact = 0, // boxcar of 1 or 2 samples: the exact window sums, in registers
     kTestGroup = 1, // per 4-sample group: group max minus the least prefix a window starts from
     kTestBlock = 2, // per thread's columns first (wide boxcars), then per group
-    kTestAll   = 3, // trapezoid: the exact test on every group
+    kTestTrap  = 3, // trapezoid: per group, half the sum of the bounds of its two boxcars
 };
 
 /** Per-width constants of the steady-state pass, built once per CTA. For a
@@ -430,8 +467,8 @@ struct WidthTest {
     int two;
     int bconst;
     int btwo;
-    float T;
-    int pad;
+    // trapezoid: the same of the inner boxcar's starts (k - W + E) and ends (k - E)
+    int iconst, itwo, econst, etwo;
 };
 
 // Loads P staged samples (16-byte aligned) as float.
@@ -631,6 +668,32 @@ __device__ __forceinline__ void group_lows(const float* gmin, int i0, bool two, 
     }
 }
 
+// The greatest of 4-column group maxima where group_lows takes the least.
+template <int NG>
+__device__ __forceinline__ void group_highs(const float* gmax, int i0, bool two, float (&hi)[NG]) {
+#pragma unroll
+    for (int g = 0; g < NG; ++g)
+        hi[g] = two ? fmaxf(gmax[i0 + g], gmax[i0 + g + 1]) : gmax[i0 + g];
+}
+
+// Whether a trapezoid of this thread's group g can exceed T. The trapezoid
+// is the mean of two boxcars, (Q[k] - Q[k - W] + Q[k - E] - Q[k - W + E]) / 2,
+// so half the sum of both ranges bounds it; the exact test's five roundings
+// and the bound's three are each at most 2^-24 of 4 max|Q|, which `margin`
+// (2^-18 max|Q|) covers. NaN: test.
+template <int NG>
+__device__ __forceinline__ void trap_bounds(const WidthTest& t, const float (&gmx)[NG], const float* gmin,
+                                            const float* gmax, float margin, float (&bound)[NG]) {
+    const int i0 = NG * static_cast<int>(threadIdx.x);
+    float low[NG], inner[NG], high[NG];
+    group_lows<NG>(gmin, i0 + t.gconst, t.two != 0, low);
+    group_lows<NG>(gmin, i0 + t.iconst, t.itwo != 0, inner);
+    group_highs<NG>(gmax, i0 + t.econst, t.etwo != 0, high);
+#pragma unroll
+    for (int g = 0; g < NG; ++g)
+        bound[g] = 0.5F * ((gmx[g] - low[g]) + (high[g] - inner[g])) + margin;
+}
+
 // The steady-state test of width 2^WI for the widths 1, 2, 4, ... (no
 // trapezoid): the same tests as the per-width table, with every offset and
 // alignment a compile-time constant (the halo is a multiple of 256, so the
@@ -696,12 +759,12 @@ __device__ __forceinline__ bool pow2_maybe(const float (&q)[P], float pm1, float
 template <int P, int NG, int WI, int WI1>
 __device__ __forceinline__ void pow2_range(uint32_t& cand, const float (&q)[P], float pm1, float pm2,
                                            const float (&gmx)[NG], float bmax, const float* gmin,
-                                           const float* tmin, int halo, const WidthTest* wt, int nw, float& m1) {
+                                           const float* tmin, int halo, const float* thr, int nw, float& m1) {
     if constexpr (WI < WI1) {
         if (WI < nw) {
-            if (pow2_maybe<P, NG, WI>(q, pm1, pm2, gmx, bmax, gmin, tmin, halo, wt[WI].T, m1))
+            if (pow2_maybe<P, NG, WI>(q, pm1, pm2, gmx, bmax, gmin, tmin, halo, thr[WI], m1))
                 cand |= 1U << WI;
-            pow2_range<P, NG, WI + 1, WI1>(cand, q, pm1, pm2, gmx, bmax, gmin, tmin, halo, wt, nw, m1);
+            pow2_range<P, NG, WI + 1, WI1>(cand, q, pm1, pm2, gmx, bmax, gmin, tmin, halo, thr, nw, m1);
         }
     }
 }
@@ -711,8 +774,11 @@ __device__ __forceinline__ void pow2_range(uint32_t& cand, const float (&q)[P], 
 // that Q[-1] = 0, and the halo's entries of gmin (per 4 columns) and tmin
 // (per P columns). Rounding is monotonic, so the least rebased value of a
 // group is its least prefix value, rebased.
+// `gmax` (null: none) takes the groups' greatest values and `qabs` the bits
+// of the greatest |value|.
 template <class S, int P>
-__device__ void scan_halo(const S* seg, int halo, int jmin, float* Q, float* gmin, float* tmin) {
+__device__ void scan_halo(const S* seg, int halo, int jmin, float* Q, float* gmin, float* tmin, float* gmax,
+                          uint32_t* qabs) {
     float* H = Q - halo;
     for (int i = threadIdx.x; i < halo; i += kThreads)
         H[i] = i < jmin ? 0.0F : ldf<S>(seg + i);
@@ -721,6 +787,13 @@ __device__ void scan_halo(const S* seg, int halo, int jmin, float* Q, float* gmi
     const float last = H[halo - 1];
     for (int j = threadIdx.x; j < halo / 4; j += kThreads)
         gmin[j] = fminf(fminf(H[4 * j], H[4 * j + 1]), fminf(H[4 * j + 2], H[4 * j + 3])) - last;
+    if (gmax != nullptr)
+        for (int j = threadIdx.x; j < halo / 4; j += kThreads) {
+            const float m = fmaxf(fmaxf(H[4 * j], H[4 * j + 1]), fmaxf(H[4 * j + 2], H[4 * j + 3])) - last;
+            gmax[j]       = m;
+            // NaN compares above everything as an integer: the bound then tests
+            atomicMax(qabs, max(__float_as_uint(fabsf(m)), __float_as_uint(fabsf(gmin[j]))));
+        }
     for (int j = threadIdx.x; j < halo / P; j += kThreads) {
         float m = H[P * j];
         for (int e = 1; e < P; ++e)
@@ -750,6 +823,8 @@ __global__ void __launch_bounds__(kThreads, FSB == 2 ? (CH == 2048 ? 4 : 3) : (C
     //   tmin   (halo + CH) / P: least Q of each thread's P columns
     //   nh     2 x nh_len: the next chunk's halo (Q, gmin, tmin and this
     //          chunk's last Q, not yet rebased), by chunk parity
+    //   gmax   trapezoid only: (halo + CH) / 4 + 4 pad, the greatest Q of each
+    //          group, and 2 x halo / 4 of the next chunk's halo
     //   bits   uint32 [nw][CH / 32]: per-width masks of the samples that fired
     //   stage  S [2][halo + CH]: the raw row segment, bulk-copied one chunk
     //          ahead (the halo columns only for the first chunk)
@@ -770,6 +845,8 @@ __global__ void __launch_bounds__(kThreads, FSB == 2 ? (CH == 2048 ? 4 : 3) : (C
     __shared__ uint32_t fired_w; // widths with a set bit in this chunk
     __shared__ float warp_tot[kThreads / 32];
     __shared__ float wtail[kThreads / 32][2]; // each warp's last two prefix values
+    __shared__ uint32_t wabs[kThreads / 32];  // trapezoid: bits of each warp's greatest |Q|
+    __shared__ uint32_t habs[2];              // and of the halo's, by chunk parity
 
     const int nw        = p.nwidths;
     const int wmax      = p.wmax;
@@ -784,12 +861,17 @@ __global__ void __launch_bounds__(kThreads, FSB == 2 ? (CH == 2048 ? 4 : 3) : (C
     float* const tmin    = gmin + seg_cols / 4 + 4;
     const int nh_len     = halo + halo / 4 + halo / P + 4;
     float* const nh0     = tmin + seg_cols / P;
-    uint32_t* const bits = reinterpret_cast<uint32_t*>(nh0 + 2 * nh_len);
+    // (the power-of-two tests are the boxcars')
+    const bool trap      = !POW2 && p.trapezoid != 0;
+    float* const gmax    = nh0 + 2 * nh_len;
+    float* const ghalo0  = gmax + seg_cols / 4 + 4;
+    uint32_t* const bits = reinterpret_cast<uint32_t*>(trap ? ghalo0 + halo / 2 : gmax);
     S* const stage0      = reinterpret_cast<S*>(bits + search_bits_words(nw, CH)); // buffer b at stage0 + b * seg_cols
     // A chunk's halo is the previous chunk's last `halo` columns, whose prefix
     // sums that chunk has: only the first chunk (or every chunk, for a halo
     // wider than a chunk) stages and scans its halo.
     const bool carry_halo = halo <= CH;
+    uint8_t* const best_w = reinterpret_cast<uint8_t*>(gmin); // across widths: CH of its 4 (halo + CH) / 4 bytes
     const int nchunks     = (p.n_valid + CH - 1) / CH;
     if (threadIdx.x == 0) {
         abort_flag = 0;
@@ -832,16 +914,23 @@ __global__ void __launch_bounds__(kThreads, FSB == 2 ? (CH == 2048 ? 4 : 3) : (C
             rc.inv[w]      = iv;
             rc.inv_or[w]   = p.inv_sigma_or[g * nw + w];
             const float T  = iv > 0.0F ? p.thresh / iv : FB_POS_INF;
-            rc.thr[w]      = T;
+            const float io = rc.inv_or[w];
+            const float To = fminf(T, io > 0.0F ? p.thresh / io : FB_POS_INF);
+            rc.thr[0][w]   = T;
+            // S/N is the product sum x inv rounded: 2^-20 is more than its and
+            // the quotient's roundings
+            rc.thr[1][w]   = isinf(To) ? To : To - fabsf(To) * 0x1p-20F;
             WidthTest t;
-            t.kind   = E > 0 ? kTestAll : W <= 2 ? kTestExact : W < 4 * P ? kTestGroup : kTestBlock;
+            t.kind   = E > 0 ? kTestTrap : W <= 2 ? kTestExact : W < 4 * P ? kTestGroup : kTestBlock;
             t.W      = W;
             t.gconst = (halo - W) >> 2;
             t.two    = ((halo - W) & 3) != 0 ? 1 : 0;
             t.bconst = (halo - W) / P;
             t.btwo   = ((halo - W) % P) != 0 ? 1 : 0;
-            t.T      = T;
-            t.pad    = 0;
+            t.iconst = (halo - W + E) >> 2;
+            t.itwo   = ((halo - W + E) & 3) != 0 ? 1 : 0;
+            t.econst = (halo - E) >> 2;
+            t.etwo   = ((halo - E) & 3) != 0 ? 1 : 0;
             wt[w]    = t;
         }
         if (threadIdx.x < nruns && !all)
@@ -930,8 +1019,11 @@ __global__ void __launch_bounds__(kThreads, FSB == 2 ? (CH == 2048 ? 4 : 3) : (C
                 break;
             const S* seg           = FS ? fs_halo : stage0 + ((cc + ci) & 1) * seg_cols;
             const bool direct_halo = ci == 0 || !carry_halo;
-            if (direct_halo)
-                scan_halo<S, P>(seg, halo, jmin, Q, gmin, tmin);
+            if (direct_halo) {
+                if (trap && threadIdx.x == 0)
+                    habs[ci & 1] = 0U; // scan_halo's first barrier orders it
+                scan_halo<S, P>(seg, halo, jmin, Q, gmin, tmin, trap ? gmax : nullptr, &habs[ci & 1]);
+            }
             // ---- prefix sums of the thread's P columns: serial, then across the
             // warp (shuffles), then across warps (one offset per warp)
             float q[P];
@@ -995,6 +1087,15 @@ __global__ void __launch_bounds__(kThreads, FSB == 2 ? (CH == 2048 ? 4 : 3) : (C
             else
                 reinterpret_cast<float2*>(gmin + halo / 4)[threadIdx.x] = make_float2(gmn[0], gmn[1]);
             tmin[halo / P + threadIdx.x] = bmin;
+            if (trap) {
+#pragma unroll
+                for (int gq = 0; gq < NG; ++gq)
+                    gmax[halo / 4 + NG * threadIdx.x + gq] = gmx[gq];
+                const uint32_t a = __reduce_max_sync(
+                    0xFFFFFFFFU, max(__float_as_uint(fabsf(bmax)), __float_as_uint(fabsf(bmin))));
+                if (lane == 0)
+                    wabs[warp] = a;
+            }
             if (lane == 31) {
                 wtail[warp][0] = q[P - 2];
                 wtail[warp][1] = q[P - 1];
@@ -1012,6 +1113,11 @@ __global__ void __launch_bounds__(kThreads, FSB == 2 ? (CH == 2048 ? 4 : 3) : (C
                     for (int gq = 0; gq < NG; ++gq)
                         nh[halo + NG * tt + gq] = gmn[gq];
                     nh[halo + halo / 4 + tt] = bmin;
+                    if (trap) {
+#pragma unroll
+                        for (int gq = 0; gq < NG; ++gq)
+                            ghalo0[(ci & 1) * (halo / 4) + NG * tt + gq] = gmx[gq];
+                    }
                     if (threadIdx.x == kThreads - 1)
                         nh[halo + halo / 4 + halo / P] = q[P - 1];
                 }
@@ -1031,6 +1137,9 @@ __global__ void __launch_bounds__(kThreads, FSB == 2 ? (CH == 2048 ? 4 : 3) : (C
                         else
                             Q[i - n - 2] = ph[halo + i - n - 2] - last;
                     }
+                    if (trap)
+                        for (int i = threadIdx.x; i < halo / 4; i += kThreads)
+                            gmax[i] = ghalo0[((ci - 1) & 1) * (halo / 4) + i] - last;
                 }
             }
             __syncthreads();
@@ -1052,16 +1161,34 @@ __global__ void __launch_bounds__(kThreads, FSB == 2 ? (CH == 2048 ? 4 : 3) : (C
                 if (threadIdx.x == 0)
                     fired_w = 0U;
             };
-            const bool fast = c0 + CH <= p.n_valid && (!p.skip_cold || rc.tile_t0 + c0 >= warm) &&
-                              (!rc.or_active || rc.tile_t0 + c0 - rc.gulp_t0 >= warm);
-            if (fast) {
-                // ---- steady state. A window sum Q[k] - Q[k - W] of a set of
-                // samples is at most their greatest Q minus the least Q their
-                // windows start from (rounding is monotonic), so a set the bound
+            const bool steady = c0 + CH <= p.n_valid && (!p.skip_cold || rc.tile_t0 + c0 >= warm) &&
+                                (!rc.or_active || rc.tile_t0 + c0 - rc.gulp_t0 >= warm);
+            const float* thr = rc.thr[steady ? 0 : 1];
+            float margin     = 0.0F; // of the trapezoid's bounds
+            if (trap) {
+                // max|Q| of the chunk and its halo: the halo's values are the
+                // previous chunk's, moved by one of them (wabs of that chunk
+                // is in habs)
+                uint32_t a = wabs[0];
+#pragma unroll
+                for (int w = 1; w < kThreads / 32; ++w)
+                    a = max(a, wabs[w]);
+                const float h = __uint_as_float(habs[ci & 1]) * (direct_halo ? 1.0F : 2.0F);
+                margin        = fmaxf(__uint_as_float(a), h) * 0x1p-18F;
+                if (isnan(h) || isnan(__uint_as_float(a)))
+                    margin = FB_POS_INF;
+                if (threadIdx.x == 0 && carry_halo)
+                    habs[(ci + 1) & 1] = a;
+            }
+            {
+                // ---- A window sum Q[k] - Q[k - W] of a set of samples is at most
+                // their greatest Q minus the least Q their windows start from (rounding is monotonic), so a set the bound
                 // clears cannot fire. Widths 1 and 2 take the exact sums in
                 // registers, the others a bound per 4-sample group (wide boxcars
                 // first one per thread); only a chunk where some test may fire
-                // stores Q and runs the exact tests.
+                // stores Q and runs the exact tests: the window sum's in steady
+                // chunks, elsewhere (cold prefix, mask change, partial chunk)
+                // the general S/N of the samples that the lower threshold left.
                 float pm1 = __shfl_up_sync(0xFFFFFFFFU, q[P - 1], 1); // Q[P t - 1]
                 float pm2 = __shfl_up_sync(0xFFFFFFFFU, q[P - 2], 1); // Q[P t - 2]
                 if (lane == 0) {
@@ -1080,12 +1207,13 @@ __global__ void __launch_bounds__(kThreads, FSB == 2 ? (CH == 2048 ? 4 : 3) : (C
                     // rounding) and is taken exactly.
                     const float qmag = fmaxf(fabsf(bmax), fabsf(bmin)) + fabsf(off);
                     float m1         = fmaxf(xmax + qmag * 0x1p-20F, q[0] - pm1);
-                    pow2_range<P, NG, 0, kMaxPow2Widths>(cand, q, pm1, pm2, gmx, bmax, gmin, tmin, halo, wt, nw, m1);
+                    pow2_range<P, NG, 0, kMaxPow2Widths>(cand, q, pm1, pm2, gmx, bmax, gmin, tmin, halo, thr, nw, m1);
                 }
                 else {
                     for (int wi = 0; wi < nw; ++wi) {
                         const WidthTest t = wt[wi];
                         bool maybe        = true;
+                        const float T     = thr[wi];
                         if (t.kind == kTestExact) {
                             float m;
                             if (t.W == 1) {
@@ -1099,14 +1227,21 @@ __global__ void __launch_bounds__(kThreads, FSB == 2 ? (CH == 2048 ? 4 : 3) : (C
                                 for (int e = 2; e < P; ++e)
                                     m = fmaxf(m, q[e] - q[e - 2]);
                             }
-                            maybe = m > t.T;
-                        } else if (t.kind != kTestAll) {
+                            maybe = m > T;
+                        } else if (t.kind == kTestTrap) {
+                            float bound[NG];
+                            trap_bounds<NG>(t, gmx, gmin, gmax, margin, bound);
+                            maybe = false;
+#pragma unroll
+                            for (int gq = 0; gq < NG; ++gq)
+                                maybe |= !(bound[gq] <= T);
+                        } else {
                             if (t.kind == kTestBlock) {
                                 const int b = static_cast<int>(threadIdx.x) + t.bconst;
                                 float lo    = tmin[b];
                                 if (t.btwo)
                                     lo = fminf(lo, tmin[b + 1]);
-                                maybe = bmax - lo > t.T;
+                                maybe = bmax - lo > T;
                             }
                             if (maybe) {
                                 float lo[NG];
@@ -1115,7 +1250,7 @@ __global__ void __launch_bounds__(kThreads, FSB == 2 ? (CH == 2048 ? 4 : 3) : (C
 #pragma unroll
                                 for (int gq = 1; gq < NG; ++gq)
                                     m = fmaxf(m, gmx[gq] - lo[gq]);
-                                maybe = m > t.T;
+                                maybe = m > T;
                             }
                         }
                         if (maybe)
@@ -1131,25 +1266,29 @@ __global__ void __launch_bounds__(kThreads, FSB == 2 ? (CH == 2048 ? 4 : 3) : (C
                 bool up = false;
                 // the exact test of group gi at width wi (sets the fired bits)
                 auto exact = [&](int gi, int wi, int W, int E, float T) {
-                    const int k    = 4 * gi;
-                    const float4 a = *reinterpret_cast<const float4*>(Q + k);
-                    const float4 b = ld4(Q, k - W);
-                    float s0, s1, s2, s3;
-                    if (E > 0) {
-                        const float4 c = ld4(Q, k - E);
-                        const float4 d = ld4(Q, k - W + E);
-                        s0 = trap_sum(a.x, b.x, c.x, d.x);
-                        s1 = trap_sum(a.y, b.y, c.y, d.y);
-                        s2 = trap_sum(a.z, b.z, c.z, d.z);
-                        s3 = trap_sum(a.w, b.w, c.w, d.w);
+                    const int k = 4 * gi;
+                    uint32_t nib;
+                    if (steady) {
+                        const float4 a = *reinterpret_cast<const float4*>(Q + k);
+                        const float4 b = ld4(Q, k - W);
+                        float s0, s1, s2, s3;
+                        if (E > 0) {
+                            const float4 c = ld4(Q, k - E);
+                            const float4 d = ld4(Q, k - W + E);
+                            s0 = trap_sum(a.x, b.x, c.x, d.x);
+                            s1 = trap_sum(a.y, b.y, c.y, d.y);
+                            s2 = trap_sum(a.z, b.z, c.z, d.z);
+                            s3 = trap_sum(a.w, b.w, c.w, d.w);
+                        } else {
+                            s0 = a.x - b.x;
+                            s1 = a.y - b.y;
+                            s2 = a.z - b.z;
+                            s3 = a.w - b.w;
+                        }
+                        nib = (s0 > T ? 1U : 0U) | (s1 > T ? 2U : 0U) | (s2 > T ? 4U : 0U) | (s3 > T ? 8U : 0U);
                     } else {
-                        s0 = a.x - b.x;
-                        s1 = a.y - b.y;
-                        s2 = a.z - b.z;
-                        s3 = a.w - b.w;
+                        nib = general_hits(p, rc, Q, c0, k, wi, row.delay);
                     }
-                    const uint32_t nib = (s0 > T ? 1U : 0U) | (s1 > T ? 2U : 0U) | (s2 > T ? 4U : 0U) |
-                                         (s3 > T ? 8U : 0U);
                     if (nib != 0U) {
                         // samples 4 gi .. 4 gi + 3: word gi / 8, nibble gi % 8
                         atomicOr(&bits[wi * (CH / 32) + (gi >> 3)], nib << ((gi & 7) * 4));
@@ -1161,41 +1300,32 @@ __global__ void __launch_bounds__(kThreads, FSB == 2 ? (CH == 2048 ? 4 : 3) : (C
                     const int wi      = __ffs(static_cast<int>(c)) - 1;
                     const WidthTest t = wt[wi];
                     const int E       = rc.E[wi];
+                    const float T     = thr[wi];
+                    const int g0      = NG * static_cast<int>(threadIdx.x);
                     if (t.kind == kTestGroup || t.kind == kTestBlock) {
                         float lo[NG];
-                        group_lows<NG>(gmin, NG * static_cast<int>(threadIdx.x) + t.gconst, t.two != 0, lo);
+                        group_lows<NG>(gmin, g0 + t.gconst, t.two != 0, lo);
 #pragma unroll
                         for (int gq = 0; gq < NG; ++gq)
-                            if (gmx[gq] - lo[gq] > t.T)
-                                exact(NG * static_cast<int>(threadIdx.x) + gq, wi, t.W, E, t.T);
+                            if (gmx[gq] - lo[gq] > T)
+                                exact(g0 + gq, wi, t.W, E, T);
+                    } else if (t.kind == kTestTrap) {
+                        float bound[NG];
+                        trap_bounds<NG>(t, gmx, gmin, gmax, margin, bound);
+#pragma unroll
+                        for (int gq = 0; gq < NG; ++gq)
+                            if (!(bound[gq] <= T))
+                                exact(g0 + gq, wi, t.W, E, T);
                     } else {
 #pragma unroll
                         for (int gq = 0; gq < NG; ++gq)
-                            exact(NG * static_cast<int>(threadIdx.x) + gq, wi, t.W, E, t.T);
+                            exact(g0 + gq, wi, t.W, E, T);
                     }
                 }
                 if (!__syncthreads_or(up)) {
                     close_runs();
                     continue;
                 }
-            } else {
-                // ---- not steady (cold prefix, mask change, partial chunk): the
-                // bit masks from the general S/N
-                store_q();
-                __syncthreads();
-                for (int j = 0; j < (CH / kThreads); ++j) {
-                    const int k = threadIdx.x + j * kThreads;
-                    for (int wi = 0; wi < nw; ++wi) {
-                        const bool hit   = snr_general(p, rc, Q, c0, k, wi, row.delay) > p.thresh;
-                        const uint32_t m = __ballot_sync(0xFFFFFFFFU, hit);
-                        if (lane == 0) {
-                            bits[wi * (CH / 32) + j * (kThreads / 32) + warp] = m;
-                            if (m != 0U)
-                                atomicOr(&fired_w, 1U << wi);
-                        }
-                    }
-                }
-                __syncthreads();
             }
             // bits now hold exactly the above-threshold samples of every width
             const uint32_t fw = fired_w;
@@ -1208,6 +1338,7 @@ __global__ void __launch_bounds__(kThreads, FSB == 2 ? (CH == 2048 ? 4 : 3) : (C
                     any_bits[wd] = m;
                 }
                 __syncthreads();
+                best_over_widths<CH>(p, rc, Q, c0, row.delay, steady, any_bits, best_w);
             }
             // Widths are independent (each has its own run state): warp w
             // walks widths w, w + 8, ..., its lanes over the chunk's samples.
@@ -1224,7 +1355,7 @@ __global__ void __launch_bounds__(kThreads, FSB == 2 ? (CH == 2048 ? 4 : 3) : (C
                             const int k = wd * 32 + __ffs(m) - 1;
                             m &= m - 1;
                             RunState r{};
-                            r.best   = snr_general(p, rc, Q, c0, k, wi, row.delay);
+                            r.best   = bit_snr(p, rc, Q, c0, k, wi, row.delay, steady);
                             r.best_w = wi;
                             r.start = r.best_t = r.last_t = rc.tile_t0 + c0 + k;
                             emit(p, row, r, &local_count);
@@ -1234,11 +1365,22 @@ __global__ void __launch_bounds__(kThreads, FSB == 2 ? (CH == 2048 ? 4 : 3) : (C
             } else if (!across) {
                 for (int wi = warp; wi < nw; wi += kThreads / 32)
                     if (((fw >> wi) & 1U) != 0U || runs[wi].open)
-                        walk_runs_warp<CH>(p, rc, Q, c0, row.delay, bits + wi * (CH / 32), wi, runs[wi], row,
-                                           &local_count);
+                        walk_runs_warp<CH>(
+                            p, rc, c0, bits + wi * (CH / 32),
+                            [&](int k, int& bw) {
+                                bw = wi;
+                                return bit_snr(p, rc, Q, c0, k, wi, row.delay, steady);
+                            },
+                            runs[wi], row, &local_count);
+            } else if (warp == 0 && (fw != 0U || runs[0].open)) {
+                walk_runs_warp<CH>(
+                    p, rc, c0, any_bits,
+                    [&](int k, int& bw) {
+                        bw = best_w[k];
+                        return Q[k];
+                    },
+                    runs[0], row, &local_count);
             }
-            if (across && warp == 0 && (fw != 0U || runs[0].open))
-                walk_runs_warp<CH>(p, rc, Q, c0, row.delay, any_bits, -1, runs[0], row, &local_count);
             __syncthreads();
         }
         if (abort_flag) {
@@ -1386,14 +1528,15 @@ void search_table(SearchSeg* segs, int n, cudaStream_t s, int32_t chunk, int32_t
     }
     const size_t es   = segs[0].fp16 ? 2 : 4;
     const size_t seg  = static_cast<size_t>(p0.halo) + chunk;
-    // Ps, gmin (+4 padding), tmin, the next chunk's halo by parity, the bit
+    // Ps, gmin (+4 padding), tmin, the next chunk's halo by parity, gmax, the bit
     // masks and the staging buffers (the kernel's layout)
     const size_t per  = static_cast<size_t>(chunk) / kThreads; // columns per thread
     const size_t nh   = static_cast<size_t>(p0.halo) + p0.halo / 4 + p0.halo / per + 4;
     // staging: two raw row segments, or (fused level step) the halo and
     // two pairs of child segments
     const size_t stage_elems = fs ? p0.halo + fsb * (2 * static_cast<size_t>(chunk) + 16 / es) : 2 * seg;
-    const size_t smem = sizeof(float) * ((4 + seg + 4) + (seg / 4 + 4) + seg / per + 2 * nh) +
+    const size_t trap = p0.trapezoid ? seg / 4 + 4 + p0.halo / 2 : 0; // gmax and its halo copies
+    const size_t smem = sizeof(float) * ((4 + seg + 4) + (seg / 4 + 4) + seg / per + 2 * nh + trap) +
                         sizeof(uint32_t) * search_bits_words(p0.nwidths, chunk) + es * stage_elems;
     const dim3 grid(static_cast<unsigned>(ctas > 0 ? std::min<int64_t>(rows, ctas) : rows));
     auto go = [&](auto kernel) {
