@@ -470,8 +470,9 @@ const float* Cleaner::execute_normalized(const uint8_t* block, SizeType bytes, S
 
     const bool short_block = valid < static_cast<SizeType>(std::max(kMinWindow, kMinBlockSamps));
     const int flip         = m_layout.df < 0.0 ? 1 : 0;
-    FB_CUDA(cudaMemsetAsync(m_out.get(), 0, capacity * m_n * sizeof(float), s));
     if (short_block && m_tail_ready) {
+        // normalize_short writes the valid samples of unmasked channels only
+        FB_CUDA(cudaMemsetAsync(m_out.get(), 0, capacity * m_n * sizeof(float), s));
         Dims d = dims(valid, m_layout.dtype);
         launch_unpack(d, raw, m_work.as<float>(), s);
         normalize_short(capacity, valid, s);

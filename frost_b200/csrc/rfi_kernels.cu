@@ -1647,119 +1647,116 @@ __global__ void __launch_bounds__(32 * (G + 1))
     }
 }
 
-constexpr int kTile = 32;
-
 // Normalise + transpose (lib/cpu/rfi_cpu.cpp:242-255): out[c][t] =
 // (work[t][c] - loc) * (scale > 0 ? 1 / scale : 1) per (window, channel),
-// masked channels zero. A block covers 32 channels and kNormSpan samples
-// in 32 x 32 tiles through shared memory; each thread keeps its channel's
-// window constants and reloads them only when its rows cross into the next
-// window.
+// masked channels and rows past the valid ones zero, so that every float of
+// out is written. A block covers 64 channels and kNormSpan samples in 64 x
+// 64 tiles through shared memory; each thread keeps its channels' window
+// constants and reloads them only when its rows cross into the next window.
+// Bound by HBM (4 bytes in and out a cell); 16 bytes a load where the
+// channels are a multiple of 4 (VL) and a store where the capacity is (VS),
+// else one float a lane and 16 in flight a thread. 1536 channels x 40 001
+// samples: 284 us with 32 x 32 tiles and four loads in flight, 133 us here; 4096 x
+// 262 144: 1750 -> 1386 us.
 constexpr int kNormSpan = 256;
+constexpr int kNT       = 64;
 
-__global__ void k_normalize(Dims d, const float* __restrict__ work, const float* __restrict__ loc,
-                            const float* __restrict__ scale, const uint8_t* __restrict__ mask,
-                            int flip, uint64_t capacity, float* __restrict__ out) {
-    __shared__ float tile[kTile][kTile + 1];
-    const uint64_t n  = d.nchans;
-    const uint64_t c0 = static_cast<uint64_t>(blockIdx.y) * kTile;
-    const uint64_t c  = c0 + threadIdx.x;
-    const bool on     = c < n && mask[c] != 0;
-    uint64_t wend     = 0;
-    float l = 0.0F, is = 1.0F;
-    const uint64_t span0 = static_cast<uint64_t>(blockIdx.x) * kNormSpan;
-    for (uint64_t t0 = span0; t0 < span0 + kNormSpan && t0 < capacity; t0 += kTile) {
-        for (int k = threadIdx.y; k < kTile; k += blockDim.y) {
-            const uint64_t t = t0 + k;
-            float v          = 0.0F;
-            if (t < d.nsamps && on) {
-                if (t >= wend) {
-                    const uint64_t w = window_of(t, d.window, d.nwin);
-                    wend             = window_end(w, d);
-                    l                = loc[w * n + c];
-                    const float sc   = scale[w * n + c];
-                    is               = sc > 0.0F ? 1.0F / sc : 1.0F;
-                }
-                v = (work[t * n + c] - l) * is;
-            }
-            tile[k][threadIdx.x] = v;
-        }
-        __syncthreads();
-        const uint64_t t = t0 + threadIdx.x;
-        if (t < capacity) {
-            for (int k = threadIdx.y; k < kTile; k += blockDim.y) {
-                const uint64_t cc = c0 + k;
-                if (cc < n) {
-                    const uint64_t dst      = flip ? n - 1 - cc : cc;
-                    out[dst * capacity + t] = tile[threadIdx.x][k];
-                }
-            }
-        }
-        __syncthreads();
-    }
-}
-
-// The same with 64 x 64 tiles and 16-byte loads and stores (nchans and the
-// output capacity multiples of 4): a thread reads 4 channels of a row and
-// writes 4 samples of a channel.
-constexpr int kNT = 64;
-
+template <bool VL, bool VS>
 __global__ void __launch_bounds__(256)
-    k_normalize4(Dims d, const float* __restrict__ work, const float* __restrict__ loc,
-                 const float* __restrict__ scale, const uint8_t* __restrict__ mask, int flip,
-                 uint64_t capacity, float* __restrict__ out) {
+    k_normalize(Dims d, const float* __restrict__ work, const float* __restrict__ loc,
+                const float* __restrict__ scale, const uint8_t* __restrict__ mask, int flip,
+                uint64_t capacity, float* __restrict__ out) {
     __shared__ float tile[kNT][kNT + 1]; // [channel][time]
+    constexpr int E     = VL ? 4 : 1;            // channels a load
+    constexpr int kRows = VL ? 16 : 4;           // rows the block loads at once
     const uint64_t n  = d.nchans;
     const uint64_t c0 = static_cast<uint64_t>(blockIdx.y) * kNT;
-    const int q       = threadIdx.x % 16; // channel quad (load) / sample quad (store)
-    const int r       = threadIdx.x / 16; // row (load) / channel (store) offset, 0..15
-    const uint64_t c  = c0 + 4 * q;
-    bool on[4];
+    const int q       = threadIdx.x % (kNT / E); // channels E q .. of the tile
+    const int r       = threadIdx.x / (kNT / E);
+    const uint64_t c  = c0 + E * q;
+    bool on[E];
 #pragma unroll
-    for (int e = 0; e < 4; ++e)
+    for (int e = 0; e < E; ++e)
         on[e] = c + e < n && mask[c + e] != 0;
     uint64_t wend = 0;
-    float l[4] = {0, 0, 0, 0}, is[4] = {1, 1, 1, 1};
+    float l[E], is[E];
+#pragma unroll
+    for (int e = 0; e < E; ++e) {
+        l[e]  = 0.0F;
+        is[e] = 1.0F;
+    }
     const uint64_t span0 = static_cast<uint64_t>(blockIdx.x) * kNormSpan;
     for (uint64_t t0 = span0; t0 < span0 + kNormSpan && t0 < capacity; t0 += kNT) {
+        float x[kNT / kRows][E];
 #pragma unroll
-        for (int pass = 0; pass < kNT / 16; ++pass) {
-            const int tl     = r + 16 * pass;
+        for (int pass = 0; pass < kNT / kRows; ++pass) {
+            const uint64_t t = t0 + r + kRows * pass;
+#pragma unroll
+            for (int e = 0; e < E; ++e)
+                x[pass][e] = 0.0F;
+            if (t < d.nsamps && c < n) {
+                if constexpr (VL) {
+                    const float4 v = *reinterpret_cast<const float4*>(work + t * n + c);
+                    x[pass][0] = v.x, x[pass][1] = v.y, x[pass][2] = v.z, x[pass][3] = v.w;
+                } else {
+                    x[pass][0] = work[t * n + c];
+                }
+            }
+        }
+#pragma unroll
+        for (int pass = 0; pass < kNT / kRows; ++pass) {
+            const int tl     = r + kRows * pass;
             const uint64_t t = t0 + tl;
-            float v[4]       = {0, 0, 0, 0};
+            float v[E];
+#pragma unroll
+            for (int e = 0; e < E; ++e)
+                v[e] = 0.0F;
             if (t < d.nsamps && c < n) {
                 if (t >= wend) {
                     const uint64_t w = window_of(t, d.window, d.nwin);
                     wend             = window_end(w, d);
 #pragma unroll
-                    for (int e = 0; e < 4; ++e) {
+                    for (int e = 0; e < E; ++e) {
                         l[e]           = loc[w * n + c + e];
                         const float sc = scale[w * n + c + e];
                         is[e]          = sc > 0.0F ? 1.0F / sc : 1.0F;
                     }
                 }
-                const float4 x = *reinterpret_cast<const float4*>(work + t * n + c);
-                const float xs[4] = {x.x, x.y, x.z, x.w};
 #pragma unroll
-                for (int e = 0; e < 4; ++e)
-                    v[e] = on[e] ? (xs[e] - l[e]) * is[e] : 0.0F;
+                for (int e = 0; e < E; ++e)
+                    v[e] = on[e] ? (x[pass][e] - l[e]) * is[e] : 0.0F;
             }
 #pragma unroll
-            for (int e = 0; e < 4; ++e)
-                tile[4 * q + e][tl] = v[e];
+            for (int e = 0; e < E; ++e)
+                tile[E * q + e][tl] = v[e];
         }
         __syncthreads();
-        const uint64_t t = t0 + 4 * q;
-        if (t < capacity) {
+        if constexpr (VS) {
+            const int tq     = threadIdx.x % 16;
+            const uint64_t t = t0 + 4 * tq;
+            if (t < capacity) {
 #pragma unroll
-            for (int pass = 0; pass < kNT / 16; ++pass) {
-                const int cl      = r + 16 * pass;
-                const uint64_t cc = c0 + cl;
-                if (cc < n) {
-                    const uint64_t dst = flip ? n - 1 - cc : cc;
-                    const float4 o = make_float4(tile[cl][4 * q], tile[cl][4 * q + 1], tile[cl][4 * q + 2],
-                                                 tile[cl][4 * q + 3]);
-                    *reinterpret_cast<float4*>(out + dst * capacity + t) = o;
+                for (int pass = 0; pass < kNT / 16; ++pass) {
+                    const int cl      = threadIdx.x / 16 + 16 * pass;
+                    const uint64_t cc = c0 + cl;
+                    if (cc < n) {
+                        const uint64_t dst = flip ? n - 1 - cc : cc;
+                        const float4 o = make_float4(tile[cl][4 * tq], tile[cl][4 * tq + 1], tile[cl][4 * tq + 2],
+                                                     tile[cl][4 * tq + 3]);
+                        *reinterpret_cast<float4*>(out + dst * capacity + t) = o;
+                    }
+                }
+            }
+        } else {
+            const int tl     = threadIdx.x % kNT;
+            const uint64_t t = t0 + tl;
+            if (t < capacity) {
+#pragma unroll
+                for (int pass = 0; pass < kNT / 4; ++pass) {
+                    const int cl      = threadIdx.x / kNT + 4 * pass;
+                    const uint64_t cc = c0 + cl;
+                    if (cc < n)
+                        out[(flip ? n - 1 - cc : cc) * capacity + t] = tile[cl][tl];
                 }
             }
         }
@@ -2089,13 +2086,11 @@ void launch_welford(const Dims& d, const float* work, const double* recip, float
 
 void launch_normalize(const Dims& d, const float* work, const float* loc, const float* scale,
                       const uint8_t* mask, int flip, uint64_t capacity, float* out, cudaStream_t s) {
-    if (d.nchans % 4 == 0 && capacity % 4 == 0) {
-        const dim3 grid(grid1(capacity, kNormSpan), grid1(d.nchans, kNT));
-        k_normalize4<<<grid, 256, 0, s>>>(d, work, loc, scale, mask, flip, capacity, out);
-    } else {
-        const dim3 grid(grid1(capacity, kNormSpan), grid1(d.nchans, kTile));
-        k_normalize<<<grid, dim3(kTile, 8), 0, s>>>(d, work, loc, scale, mask, flip, capacity, out);
-    }
+    const dim3 grid(grid1(capacity, kNormSpan), grid1(d.nchans, kNT));
+    const bool vl = d.nchans % 4 == 0, vs = capacity % 4 == 0;
+    const auto k  = vl ? (vs ? &k_normalize<true, true> : &k_normalize<true, false>)
+                       : (vs ? &k_normalize<false, true> : &k_normalize<false, false>);
+    k<<<grid, 256, 0, s>>>(d, work, loc, scale, mask, flip, capacity, out);
     FB_COUNT_LAUNCH();
 }
 

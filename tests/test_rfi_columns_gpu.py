@@ -163,3 +163,25 @@ def test_golden_digests(name):
     for step, (block, nsamps) in enumerate(blocks):
         assert digest(gpu.execute_normalized(block, nsamps)) == golden[step]["out_sha256"]
         assert digest(gpu.channel_mask()) == golden[step]["mask_sha256"]
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("nchans,capacity,valid", [(64, 256, 256), (64, 257, 131), (65, 320, 320), (67, 321, 65),
+                                                   (4, 64, 64), (130, 1023, 1000)])
+def test_normalize_writes_every_cell(nchans, capacity, valid):
+    """Vector and scalar loads and stores of the transpose; masked channels
+    and rows past the valid ones are zero in a buffer that held other data
+    (a second, shorter block after a whole one)."""
+    from frost_b200.rfi import RFICleaner
+    rng = np.random.default_rng(nchans + capacity)
+    x = samples(rng, capacity, nchans, DataType.FLOAT32)
+    cfg = RfiConfig.quiet()
+    cfg.zap_chans = [(1, 1)]
+    gpu = RFICleaner(cfg, BlockLayout(nchans, capacity, DataType.FLOAT32, 2.0 ** -10, 1400.0, -1.0), 32.0)
+    gpu.execute_normalized(pack(x + 1, DataType.FLOAT32))
+    got = gpu.execute_normalized(pack(x, DataType.FLOAT32), valid)
+    level, scale = bandpass(x[:valid])
+    want = np.zeros((nchans, capacity), np.float32)
+    want[:, :valid] = ((x[:valid] - level) * (np.float32(1) / scale)).T
+    want[1] = 0
+    assert np.array_equal(got.view(np.uint32), want[::-1].view(np.uint32))
