@@ -182,11 +182,12 @@ __global__ void k_sample_rows(Dims d, const uint8_t* __restrict__ raw, float* __
 // level), so its groups are independent: k_remedian evaluates it in
 // parallel. One CTA covers 32 channels (a lane each) of one window; each
 // warp reduces 125-row blocks (three tree levels in registers) to one value
-// per channel, and warp 0 finishes the tree over the <= 25 block values.
-// Pass 1 (ABS false) writes the level to loc and a flat flag (every sampled
-// value of the channel compares equal) to inv; pass 2 (ABS true) the scale,
-// remedian(|x - level|) x 1.4826, to scale (lib/cpu/spectra_cpu.cpp:73-130).
-constexpr int kRemedianWarps = 8;
+// per channel, and warp 0 finishes the tree over the <= 25 block values. The
+// level goes to loc and a flat flag (every sampled value of the channel
+// compares equal) to inv; a second sweep takes the scale, remedian(|x -
+// level|) x 1.4826 (lib/cpu/spectra_cpu.cpp:73-130). 25 warps, one a block,
+// where channel groups are few (load latency bounds them: 64 channels 33 +
+// 20 us with 8 warps and two launches, 16 here), else 8.
 
 // The remedian of 25 values p[0], p[stride], ... (medians of five
 // consecutive values, then their median): the 25 loads are issued together
@@ -254,31 +255,17 @@ __device__ __forceinline__ float remedian125(const float* __restrict__ p, uint64
     return median5(a, b, c, d, e);
 }
 
-template <bool ABS>
-__global__ void __launch_bounds__(32 * kRemedianWarps)
-    k_remedian(Dims d, const float* __restrict__ samples, float* __restrict__ loc, float* __restrict__ scale,
-               float* __restrict__ flat_out) {
-    __shared__ float part[25][32];
-    __shared__ float plo[kRemedianWarps][32], phi[kRemedianWarps][32];
+/** The 32 channels' remedian over the window's sampled rows (ABS: of |x -
+ * level|) in warp 0's lanes; lo, hi the range of this warp's values. */
+template <bool ABS, int W>
+__device__ __forceinline__ float remedian_rows(const float* __restrict__ src, uint64_t n, int levels, bool in,
+                                               float level, float (&part)[25][32], float& lo, float& hi) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const uint64_t n = d.nchans;
-    const uint64_t c = static_cast<uint64_t>(blockIdx.x) * 32 + lane;
-    const uint64_t w = blockIdx.y;
-    const bool in    = c < n;
-    const uint64_t len = window_end(w, d) - window_begin(w, d.window);
-    const uint64_t m   = largest_power_of_five_leq(len < kMaxBandpassRows ? len : kMaxBandpassRows);
-    int levels = 0;
-    for (uint64_t q = m; q > 1; q /= 5)
-        ++levels;
     const int kb       = levels < 3 ? levels : 3; // tree levels inside a block
     const int up       = levels - kb;             // levels over the blocks (0..2)
     const int nblk     = up == 0 ? 1 : up == 1 ? 5 : 25;
-    const uint64_t blk = kb == 1 ? 5 : kb == 2 ? 25 : 125;
-    const uint64_t o   = w * n + c;
-    const float level  = (ABS && in) ? loc[o] : 0.0F;
-    const float* src   = samples + w * kMaxBandpassRows * n + (in ? c : 0);
-    float lo = FLT_MAX, hi = -FLT_MAX;
-    for (int b = warp; b < nblk; b += kRemedianWarps) {
+    const uint64_t blk = kb == 1 ? 5 : kb == 2 ? 25 : 125; // a window has 5 rows or more
+    for (int b = warp; b < nblk; b += W) {
         const float* p = src + static_cast<uint64_t>(b) * blk * n;
         float v        = 0.0F;
         if (in) {
@@ -290,19 +277,11 @@ __global__ void __launch_bounds__(32 * kRemedianWarps)
         }
         part[b][lane] = v;
     }
-    if constexpr (!ABS) {
-        plo[warp][lane] = lo;
-        phi[warp][lane] = hi;
-    }
     __syncthreads();
-    if (warp != 0 || !in)
-        return;
-    float r;
-    if (up == 0) {
-        r = part[0][lane];
-    } else if (up == 1) {
+    float r = part[0][lane];
+    if (warp == 0 && up == 1) {
         r = median5(part[0][lane], part[1][lane], part[2][lane], part[3][lane], part[4][lane]);
-    } else {
+    } else if (warp == 0 && up == 2) {
         float v[5];
 #pragma unroll
         for (int j = 0; j < 5; ++j)
@@ -310,18 +289,47 @@ __global__ void __launch_bounds__(32 * kRemedianWarps)
                            part[5 * j + 3][lane], part[5 * j + 4][lane]);
         r = median5(v[0], v[1], v[2], v[3], v[4]);
     }
-    if constexpr (ABS) {
-        scale[o] = r * kMadToStd;
-    } else {
-        float a = plo[0][lane], z = phi[0][lane];
+    return r;
+}
+
+template <int W>
+__global__ void __launch_bounds__(32 * W)
+    k_remedian(Dims d, const float* __restrict__ samples, float* __restrict__ loc, float* __restrict__ scale,
+               float* __restrict__ flat_out) {
+    __shared__ float part[25][32];
+    __shared__ float plo[W][32], phi[W][32];
+    __shared__ float level_of[32];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const uint64_t n = d.nchans;
+    const uint64_t c = static_cast<uint64_t>(blockIdx.x) * 32 + lane;
+    const uint64_t w = blockIdx.y;
+    const bool in    = c < n;
+    const uint64_t len = window_end(w, d) - window_begin(w, d.window);
+    const uint64_t m   = largest_power_of_five_leq(len < kMaxBandpassRows ? len : kMaxBandpassRows);
+    int levels = 0;
+    for (uint64_t q = m; q > 1; q /= 5)
+        ++levels;
+    const uint64_t o = w * n + c;
+    const float* src = samples + w * kMaxBandpassRows * n + (in ? c : 0);
+    float lo = FLT_MAX, hi = -FLT_MAX, ignored_lo = 0.0F, ignored_hi = 0.0F;
+    const float level = remedian_rows<false, W>(src, n, levels, in, 0.0F, part, lo, hi);
+    plo[warp][lane]   = lo;
+    phi[warp][lane]   = hi;
+    if (warp == 0)
+        level_of[lane] = level;
+    __syncthreads();
+    const float r = remedian_rows<true, W>(src, n, levels, in, level_of[lane], part, ignored_lo, ignored_hi);
+    if (warp != 0 || !in)
+        return;
+    float a = plo[0][lane], z = phi[0][lane];
 #pragma unroll
-        for (int k = 1; k < kRemedianWarps; ++k) {
-            a = fminf(a, plo[k][lane]);
-            z = fmaxf(z, phi[k][lane]);
-        }
-        loc[o]      = r;
-        flat_out[o] = z > a ? 0.0F : 1.0F;
+    for (int k = 1; k < W; ++k) {
+        a = fminf(a, plo[k][lane]);
+        z = fmaxf(z, phi[k][lane]);
     }
+    loc[o]      = level;
+    flat_out[o] = z > a ? 0.0F : 1.0F;
+    scale[o]    = r * kMadToStd;
 }
 
 // The clipped refinement of the bandpass (lib/cpu/bandpass_kernels.hpp:17-76)
@@ -1013,6 +1021,22 @@ struct ScanColAcc {
     }
 };
 
+// Without zdot and Kadane the column scan only looks for the range of
+// unmeasured cells: whether any of the block's active channels has one in the
+// chunk's windows. A whole pass over the raw block is left out where none
+// has (64 channels x 4096 samples: 71 us of a 450 us clean, 744 4-bit
+// channels x 229 009: 662 us of 3430; the check takes 3).
+__device__ __forceinline__ bool block_has_unmeasured(const Dims& d, const float* __restrict__ inv, uint64_t c,
+                                                     bool active, uint64_t t0, uint64_t t1) {
+    bool some = false;
+    if (active && t0 < t1) {
+        const uint64_t w1 = window_of(t1 - 1, d.window, d.nwin);
+        for (uint64_t w = window_of(t0, d.window, d.nwin); w <= w1; ++w)
+            some |= inv[w * d.nchans + c] == 0.0F;
+    }
+    return __syncthreads_or(some) != 0;
+}
+
 template <int D>
 __global__ void k_scan_cols(Dims d, const uint8_t* __restrict__ raw, const float* __restrict__ loc,
                             const float* __restrict__ inv, const uint8_t* __restrict__ mask,
@@ -1023,12 +1047,14 @@ __global__ void k_scan_cols(Dims d, const uint8_t* __restrict__ raw, const float
                             KadaneState* __restrict__ kp_out, KadaneState* __restrict__ kn_out) {
     const uint64_t c = blockIdx.x * static_cast<uint64_t>(blockDim.x) + threadIdx.x;
     const uint64_t k = blockIdx.y;
-    if (c >= d.nchans)
+    const bool in    = c < d.nchans;
+    const uint64_t t0 = k * d.chunk;
+    const uint64_t t1 = (t0 + d.chunk < d.nsamps) ? t0 + d.chunk : d.nsamps;
+    const bool walk = zdot || kchan || block_has_unmeasured(d, inv, c, in && mask[c] != 0, t0, t1);
+    if (!in)
         return;
     ScanColAcc acc{&d, loc, inv, clip_mean, clip_inv_std, s_keep_d, c, clip, zdot, kchan};
-    if (mask[c] != 0) {
-        const uint64_t t0 = k * d.chunk;
-        const uint64_t t1 = (t0 + d.chunk < d.nsamps) ? t0 + d.chunk : d.nsamps;
+    if (walk && mask[c] != 0) {
         if (t0 < t1)
             acc.begin(t0);
         for (uint64_t tb = t0; tb < t1; tb += kBlock) {
@@ -1066,6 +1092,11 @@ __global__ void __launch_bounds__(kStageChans)
     ScanColAcc acc{&d, loc, inv, clip_mean, clip_inv_std, s_keep_d, c, clip, zdot, kchan};
     const uint64_t t0   = k * d.chunk;
     const uint64_t t1   = (t0 + d.chunk < d.nsamps) ? t0 + d.chunk : d.nsamps;
+    if (!zdot && !kchan && !block_has_unmeasured(d, inv, c, active, t0, t1)) {
+        if (in)
+            acc.store(k, cmin_out, cmax_out, zs_out, kp_out, kn_out);
+        return;
+    }
     const uint64_t off  = c0 * kBitsOf<D> / 8;
     const uint64_t left = d.row_bytes - off;
     const int copy      = static_cast<int>(left < static_cast<uint64_t>(seg_bytes) ? left : seg_bytes);
@@ -1089,22 +1120,37 @@ __global__ void __launch_bounds__(kStageChans)
         acc.store(k, cmin_out, cmax_out, zs_out, kp_out, kn_out);
 }
 
-// Per channel, in chunk order: the block min/max of unmeasured cells, the
-// zdot sums and the combined Kadane-along-time states
-// (lib/cpu/rfi_cpu.cpp:352-366, 413-466).
-__global__ void k_combine_chunks(Dims d, int zdot, int kchan, const float* __restrict__ cmin,
-                                 const float* __restrict__ cmax, const ZdotSums* __restrict__ zs,
-                                 const KadaneState* __restrict__ kp,
-                                 const KadaneState* __restrict__ kn, float* __restrict__ lo_out,
-                                 float* __restrict__ hi_out, ZdotSums* __restrict__ zs_out,
-                                 Run* __restrict__ kp_best, Run* __restrict__ kn_best) {
-    const uint64_t c = blockIdx.x * static_cast<uint64_t>(blockDim.x) + threadIdx.x;
+// Per channel, in chunk order: the block min/max of unmeasured cells and the
+// zdot sums (blockIdx.y 0), the combined Kadane-along-time states of u (1)
+// and of -u (2), and of those the best run (lib/cpu/rfi_cpu.cpp:352-366,
+// 413-466). A chain of up to 64 states a channel, bound by their loads'
+// latency: a warp a CTA, one kind of state each, the next state read while
+// one is combined. 1024 channels, 64 chunks: 31 us (209 with all three in one
+// thread's turn).
+__global__ void __launch_bounds__(32)
+    k_combine_chunks(Dims d, int zdot, const float* __restrict__ cmin, const float* __restrict__ cmax,
+                     const ZdotSums* __restrict__ zs, const KadaneState* __restrict__ kp,
+                     const KadaneState* __restrict__ kn, float* __restrict__ lo_out, float* __restrict__ hi_out,
+                     ZdotSums* __restrict__ zs_out, Run* __restrict__ kp_best, Run* __restrict__ kn_best) {
+    const uint64_t c = blockIdx.x * 32ULL + threadIdx.x;
     if (c >= d.nchans)
         return;
     const uint64_t n = d.nchans;
+    if (blockIdx.y != 0) {
+        const KadaneState* in = blockIdx.y == 1 ? kp : kn;
+        KadaneState sum = KadaneState::make(), next = in[c];
+        for (uint64_t k = 0; k < d.nchunks; ++k) {
+            const KadaneState now = next;
+            if (k + 1 < d.nchunks)
+                next = in[(k + 1) * n + c];
+            sum = KadaneState::combine(sum, now);
+        }
+        (blockIdx.y == 1 ? kp_best : kn_best)[c] = sum.best;
+        return;
+    }
     float lo = FLT_MAX, hi = -FLT_MAX;
     ZdotSums s{0, 0, 0, 0, 0};
-    KadaneState pos = KadaneState::make(), neg = KadaneState::make();
+#pragma unroll 4
     for (uint64_t k = 0; k < d.nchunks; ++k) {
         lo = smin(lo, cmin[k * n + c]);
         hi = smax(hi, cmax[k * n + c]);
@@ -1116,19 +1162,11 @@ __global__ void k_combine_chunks(Dims d, int zdot, int kchan, const float* __res
             s.sss += p.sss;
             s.szs += p.szs;
         }
-        if (kchan) {
-            pos = KadaneState::combine(pos, kp[k * n + c]);
-            neg = KadaneState::combine(neg, kn[k * n + c]);
-        }
     }
     lo_out[c] = lo;
     hi_out[c] = hi;
     if (zdot)
         zs_out[c] = s;
-    if (kchan) {
-        kp_best[c] = pos.best;
-        kn_best[c] = neg.best;
-    }
 }
 
 // ---- apply ------------------------------------------------------------------
@@ -1862,11 +1900,12 @@ void launch_sample_rows(const Dims& d, const uint8_t* raw, float* samples, cudaS
 
 void launch_bandpass(const Dims& d, const float* samples, float* loc, float* scale, float* inv,
                      uint32_t* unmeasured, cudaStream_t s) {
-    // level and flat flag, then the scale, then the clipped refinement
+    // level, flat flag and scale, then the clipped refinement
     const dim3 grid(grid1(d.nchans, 32), static_cast<unsigned>(d.nwin));
-    k_remedian<false><<<grid, 32 * kRemedianWarps, 0, s>>>(d, samples, loc, scale, inv);
-    FB_COUNT_LAUNCH();
-    k_remedian<true><<<grid, 32 * kRemedianWarps, 0, s>>>(d, samples, loc, scale, inv);
+    if (cols::few_groups(static_cast<uint64_t>(grid.x) * grid.y))
+        k_remedian<25><<<grid, 32 * 25, 0, s>>>(d, samples, loc, scale, inv);
+    else
+        k_remedian<8><<<grid, 32 * 8, 0, s>>>(d, samples, loc, scale, inv);
     FB_COUNT_LAUNCH();
     auto refine = [&](auto u, auto groups) {
         constexpr int U = decltype(u)::value, G = decltype(groups)::value;
@@ -1967,9 +2006,8 @@ void launch_scan_cols(const Dims& d, const uint8_t* raw, const float* loc, const
                                  chunk_kneg, g.seg_bytes, g.rows));
     }
     FB_COUNT_LAUNCH();
-    k_combine_chunks<<<grid1(d.nchans, 128), 128, 0, s>>>(d, zdot, kchan, chunk_min, chunk_max,
-                                                          chunk_zdot, chunk_kpos, chunk_kneg, lo,
-                                                          hi, zdot_sum, kpos_best, kneg_best);
+    k_combine_chunks<<<dim3(grid1(d.nchans, 32), kchan ? 3 : 1), 32, 0, s>>>(
+        d, zdot, chunk_min, chunk_max, chunk_zdot, chunk_kpos, chunk_kneg, lo, hi, zdot_sum, kpos_best, kneg_best);
     FB_COUNT_LAUNCH();
 }
 
