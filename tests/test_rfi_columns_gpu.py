@@ -185,3 +185,25 @@ def test_normalize_writes_every_cell(nchans, capacity, valid):
     want[:, :valid] = ((x[:valid] - level) * (np.float32(1) / scale)).T
     want[1] = 0
     assert np.array_equal(got.view(np.uint32), want[::-1].view(np.uint32))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("nsamps", [64, 1001, 8193, 400001])
+def test_dropout_cut_is_the_exact_median(nsamps):
+    """Rows whose spread is below 0.97 of the median row spread (one rank of
+    a series shorter than a CTA's share to one too long for shared memory),
+    and their neighbours, are flagged."""
+    from frost_b200.rfi import RFICleaner
+    nchans, fraction = 8, 0.97
+    rng = np.random.default_rng(nsamps)
+    x = np.clip(np.rint(rng.normal(120, 12, (nsamps, nchans))), 0, 255)
+    cfg = RfiConfig.quiet()
+    cfg.dropout.enabled = True
+    cfg.dropout.min_std_fraction = fraction
+    gpu = RFICleaner(cfg, BlockLayout(nchans, nsamps, DataType.UINT8, 2.0 ** -10, 1400.0, 1.0), 4096.0)
+    gpu.execute_normalized(pack(x, DataType.UINT8))
+    mean = x.sum(1) / nchans
+    spread = np.sqrt(np.maximum(np.square(x).sum(1) / nchans - mean * mean, 0)).astype(np.float32)
+    low = spread < np.float32(fraction) * np.sort(spread)[nsamps // 2]
+    want = low | np.append(low[1:], False) | np.insert(low[:-1], 0, False)
+    assert np.array_equal(gpu.time_flags(nsamps).astype(bool), want)
