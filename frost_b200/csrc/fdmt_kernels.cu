@@ -927,25 +927,83 @@ __global__ void __launch_bounds__(256)
         dst[r * dpitch + c] = src[r * spitch + c];
     }
 }
+
+// The same from rows that start at any even byte (a ragged gulp's last
+// columns): the destination's 16-byte vectors put together from aligned
+// words, shifted by two bytes where a row starts inside one. Words are read
+// only where they hold bytes of the row.
+__global__ void __launch_bounds__(256)
+    k_copy_rows_shifted(uint4* __restrict__ dst, int64_t dpitch, const unsigned char* __restrict__ src,
+                        int64_t spitch, uint32_t w, uint32_t n) {
+    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+        const uint32_t r = i / w, c = i - r * w;
+        const unsigned char* a = src + r * spitch + c * 16;
+        const uint32_t m       = static_cast<uint32_t>(reinterpret_cast<uintptr_t>(a) & 3U);
+        const uint32_t* v      = reinterpret_cast<const uint32_t*>(a - m);
+        uint32_t x[5];
+#pragma unroll
+        for (int k = 0; k < 4; ++k)
+            x[k] = v[k];
+        x[4] = m != 0 ? v[4] : 0U;
+        dst[r * dpitch + c] = make_uint4(__funnelshift_r(x[0], x[1], 8 * m), __funnelshift_r(x[1], x[2], 8 * m),
+                                         __funnelshift_r(x[2], x[3], 8 * m), __funnelshift_r(x[3], x[4], 8 * m));
+    }
+}
+
+// dst[r][0 .. w) = src[r][0 .. w) in floats (the input history's few columns).
+__global__ void __launch_bounds__(256)
+    k_copy_rows4(float* __restrict__ dst, int64_t dpitch, const float* __restrict__ src, int64_t spitch, uint32_t w,
+                 uint32_t n) {
+    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+        const uint32_t r = i / w, c = i - r * w;
+        dst[r * dpitch + c] = src[r * spitch + c];
+    }
+}
+
+unsigned copy_blocks(size_t n) {
+    int dev = 0, sms = 0;
+    FB_CUDA(cudaGetDevice(&dev));
+    FB_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+    return static_cast<unsigned>(std::min<size_t>((n + 255) / 256, static_cast<size_t>(sms) * 8));
+}
+
+void copy_floats(float* dst, size_t dpitch, const float* src, size_t spitch, size_t width, size_t rows,
+                 cudaStream_t s) {
+    const size_t n = width * rows;
+    if (n == 0)
+        return;
+    if (n > 0x7FFFFFFFU) {
+        FB_CUDA(cudaMemcpy2DAsync(dst, dpitch * sizeof(float), src, spitch * sizeof(float), width * sizeof(float),
+                                  rows, cudaMemcpyDeviceToDevice, s));
+        return;
+    }
+    k_copy_rows4<<<copy_blocks(n), 256, 0, s>>>(dst, static_cast<int64_t>(dpitch), src, static_cast<int64_t>(spitch),
+                                                static_cast<uint32_t>(width), static_cast<uint32_t>(n));
+    FB_LAUNCH_CHECK();
+}
 } // namespace
 
+// A ragged gulp's rows are copied by a kernel too: a 2-D memcpy of them took
+// 0.32 of the 4.0 ms of a 1000-channel search of 50 001 samples (3.75 now).
 void copy_rows(void* dst, size_t dpitch, const void* src, size_t spitch, size_t width, size_t rows,
                cudaStream_t s) {
     if (rows == 0 || width == 0)
         return;
-    const uintptr_t bits = reinterpret_cast<uintptr_t>(dst) | reinterpret_cast<uintptr_t>(src) | dpitch | spitch | width;
-    const size_t n = rows * (width / 16);
-    if (bits % 16 != 0 || n > 0x7FFFFFFFU) {
+    const uintptr_t to   = reinterpret_cast<uintptr_t>(dst) | dpitch | width;
+    const uintptr_t from = reinterpret_cast<uintptr_t>(src) | spitch;
+    const size_t n       = rows * (width / 16);
+    if (to % 16 != 0 || from % 2 != 0 || n > 0x7FFFFFFFU) {
         FB_CUDA(cudaMemcpy2DAsync(dst, dpitch, src, spitch, width, rows, cudaMemcpyDeviceToDevice, s));
         return;
     }
-    int dev = 0, sms = 0;
-    FB_CUDA(cudaGetDevice(&dev));
-    FB_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-    const size_t blocks = std::min<size_t>((n + 255) / 256, static_cast<size_t>(sms) * 8);
-    k_copy_rows16<<<static_cast<unsigned>(blocks), 256, 0, s>>>(
-        static_cast<uint4*>(dst), static_cast<int64_t>(dpitch / 16), static_cast<const uint4*>(src),
-        static_cast<int64_t>(spitch / 16), static_cast<uint32_t>(width / 16), static_cast<uint32_t>(n));
+    if (from % 16 != 0)
+        k_copy_rows_shifted<<<copy_blocks(n), 256, 0, s>>>(
+            static_cast<uint4*>(dst), static_cast<int64_t>(dpitch / 16), static_cast<const unsigned char*>(src),
+            static_cast<int64_t>(spitch), static_cast<uint32_t>(width / 16), static_cast<uint32_t>(n));
+    else
+        k_copy_rows16<<<copy_blocks(n), 256, 0, s>>>(
+            static_cast<uint4*>(dst), static_cast<int64_t>(dpitch / 16), static_cast<const uint4*>(src),
+            static_cast<int64_t>(spitch / 16), static_cast<uint32_t>(width / 16), static_cast<uint32_t>(n));
     FB_LAUNCH_CHECK();
 }
 
@@ -972,20 +1030,16 @@ void launch_save_input_history(const float* wf, int64_t pitch, int64_t t0, int32
                                cudaStream_t s) {
     if (hist_len == 0)
         return;
-    const size_t es = sizeof(float);
+    const size_t len = static_cast<size_t>(hist_len), valid = static_cast<size_t>(n_valid), step = static_cast<size_t>(pitch);
     if (n_valid >= hist_len) {
-        FB_CUDA(cudaMemcpy2DAsync(hist, hist_len * es, wf + t0 + n_valid - hist_len, pitch * es,
-                                  hist_len * es, nchans, cudaMemcpyDeviceToDevice, s));
+        copy_floats(hist, len, wf + t0 + n_valid - hist_len, step, len, static_cast<size_t>(nchans), s);
         return;
     }
     // Keep the newest hist_len - n_valid old samples, then append the tile.
-    const int32_t keep = hist_len - n_valid;
-    FB_CUDA(cudaMemcpy2DAsync(scratch, hist_len * es, hist + n_valid, hist_len * es, keep * es,
-                              nchans, cudaMemcpyDeviceToDevice, s));
-    if (n_valid > 0)
-        FB_CUDA(cudaMemcpy2DAsync(scratch + keep, hist_len * es, wf + t0, pitch * es, n_valid * es,
-                                  nchans, cudaMemcpyDeviceToDevice, s));
-    FB_CUDA(cudaMemcpyAsync(hist, scratch, static_cast<size_t>(nchans) * hist_len * es,
+    const size_t keep = len - valid;
+    copy_floats(scratch, len, hist + n_valid, len, keep, static_cast<size_t>(nchans), s);
+    copy_floats(scratch + keep, len, wf + t0, step, valid, static_cast<size_t>(nchans), s);
+    FB_CUDA(cudaMemcpyAsync(hist, scratch, static_cast<size_t>(nchans) * len * sizeof(float),
                             cudaMemcpyDeviceToDevice, s));
 }
 
