@@ -83,6 +83,9 @@ struct Seg {
 
 void launch_iota(u32* v, size_t n, cudaStream_t s);
 
+/** Pairs one CTA sorts by itself (radix_sort, in place). */
+constexpr int kSmallSort = 8192;
+
 /** Stable sort of (keys, vals) by the low `bits` bits of keys; returns
  * through the references the buffers holding the result (ping-ponged with
  * the *_alt buffers). `hist` holds 256 * ceil(n / kTile) words. */

@@ -1178,7 +1178,7 @@ void Engine::collect(cudaStream_t s) {
         launch_cand_keys(cands, n, spec, keys, vals, s);
         pp::radix_sort(keys, vals, keys_alt, vals_alt, n, key_bits, m_sort_hist.as<uint32_t>(), s);
         launch_cand_gather(cands, vals, n, m_cands_sorted.as<frost_candidate>(), s);
-        m_launches += 2 + 3 * static_cast<uint64_t>((key_bits + 7) / 8);
+        m_launches += 2 + (n <= pp::kSmallSort ? 1 : 3 * static_cast<uint64_t>((key_bits + 7) / 8));
         FB_CUDA(cudaMemcpyAsync(m_results.data(), m_cands_sorted.get(), n * sizeof(frost_candidate),
                                 cudaMemcpyDeviceToHost, s));
         FB_CUDA(cudaStreamSynchronize(s));
@@ -1215,15 +1215,12 @@ uint64_t Engine::frontier() {
     const SizeType nruns = m_cfg.peak_mode == FROST_PEAK_ACROSS_WIDTHS ? 1 : m_plan.widths().size();
     if (m_cfg.peak_mode == FROST_PEAK_ALL)
         return m_samples;
-    std::vector<RunState> runs(m_nsearch * nruns);
+    auto* f = m_frontier.as<unsigned long long>();
+    launch_frontier(m_carry.as<RunState>(), static_cast<int64_t>(m_nsearch * nruns), m_samples, f, m_stream);
+    unsigned long long out = 0;
+    FB_CUDA(cudaMemcpyAsync(&out, f, sizeof(out), cudaMemcpyDeviceToHost, m_stream));
     FB_CUDA(cudaStreamSynchronize(m_stream));
-    if (!runs.empty())
-        FB_CUDA(cudaMemcpy(runs.data(), m_carry.get(), runs.size() * sizeof(RunState), cudaMemcpyDeviceToHost));
-    uint64_t f = m_samples;
-    for (const auto& r : runs)
-        if (r.open)
-            f = std::min<uint64_t>(f, static_cast<uint64_t>(r.start));
-    return f;
+    return out;
 }
 
 frost_search_info Engine::info() const {

@@ -143,6 +143,10 @@ void launch_variance(const SearchRow* rows, const PlaneInfo* planes, const int64
                      const uint8_t* mask_or, double* var, float* inv_sigma, float* inv_sigma_or,
                      cudaStream_t s);
 
+/** *out = the earliest start of an open run of carry[0, n), else `samples`. */
+void launch_frontier(const RunState* carry, int64_t n, unsigned long long samples, unsigned long long* out,
+                     cudaStream_t s);
+
 /** Emits every open run as a candidate and closes it (drain). */
 void launch_flush_runs(const SearchParams& p, int64_t nrows, cudaStream_t s);
 
