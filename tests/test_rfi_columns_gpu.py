@@ -207,3 +207,32 @@ def test_dropout_cut_is_the_exact_median(nsamps):
     low = spread < np.float32(fraction) * np.sort(spread)[nsamps // 2]
     want = low | np.append(low[1:], False) | np.insert(low[:-1], 0, False)
     assert np.array_equal(gpu.time_flags(nsamps).astype(bool), want)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("nchans,nsamps", [(7, 300), (35, 1025), (131, 2050), (1501, 1100), (1504, 2049)])
+@pytest.mark.parametrize("zdot", [False, True])
+def test_scans_do_not_depend_on_the_sample_type(nchans, nsamps, zdot):
+    """Kadane across frequency and along time and the zdot sums of the same
+    values as uint8, uint16 and float32 (rows of any pitch, shifted and whole
+    vectors), with masked channels, an unmeasured one and runs of both signs."""
+    from frost_b200.rfi import RFICleaner
+    rng = np.random.default_rng(nchans + nsamps)
+    x = rng.normal(120, 12, (nsamps, nchans))
+    x[nsamps // 3:nsamps // 3 + 4, nchans // 4:nchans // 2 + 1] += 60
+    x[nsamps // 2:nsamps // 2 + 4, nchans // 3:] -= 50
+    x[nsamps // 4:nsamps // 4 + 120, nchans // 2] += 25
+    x[:nsamps // 2, nchans - 1] = 120
+    x = np.clip(np.rint(x), 0, 255)
+    cfg = RfiConfig()
+    cfg.kadane_channel.enabled = cfg.kadane_spectrum.enabled = True
+    cfg.kadane_channel.min_duration, cfg.kadane_spectrum.min_bandwidth = 0.02, 2.0
+    cfg.zero_dm = ZeroDMMode.ZDOT if zdot else ZeroDMMode.OFF
+    cfg.zap_chans = [(2, 2)]
+    out = []
+    for dtype in (DataType.UINT8, DataType.UINT16, DataType.FLOAT32):
+        gpu = RFICleaner(cfg, BlockLayout(nchans, nsamps, dtype, 2.0 ** -10, 1400.0, 1.0), 500 * 2.0 ** -10)
+        rep = (digest(gpu.execute_normalized(pack(x, dtype))), gpu.report())
+        out.append((rep[0],) + tuple(rep[1][k] for k in ("samps_kadane", "cells_kadane_spectrum",
+                                                         "cells_kadane_channel", "samps_broad", "chans_dead")))
+    assert out[0] == out[1] == out[2]
