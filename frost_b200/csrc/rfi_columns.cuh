@@ -128,15 +128,20 @@ template <int BITS, int U, int H, int S, bool SIDE = false> struct Ring {
                 const uint8_t* a    = s + static_cast<uint64_t>(r) * pitch + u * U;
                 const uint64_t step = kPer * pitch;
                 if (u * U < copy) {
-#pragma unroll 8
-                    for (int j = 0; j < H / kPer; ++j) {
-                        if (r + j * kPer < nr) {
-                            if constexpr (U == 16)
-                                stage::cp_async16(dst + (lane + 32 * j) * 16, a);
-                            else
-                                cp_async4(dst + (lane + 32 * j) * 4, a, 4);
-                        }
+                    auto put = [&](int j) {
+                        if constexpr (U == 16)
+                            stage::cp_async16(dst + (lane + 32 * j) * 16, a);
+                        else
+                            cp_async4(dst + (lane + 32 * j) * 4, a, 4);
                         a += step;
+                    };
+                    if (nr == H) { // a whole stage
+#pragma unroll 16
+                        for (int j = 0; j < H / kPer; ++j)
+                            put(j);
+                    } else {
+                        for (int j = 0; r + j * kPer < nr; ++j)
+                            put(j);
                     }
                 }
             } else {
