@@ -512,14 +512,9 @@ const float* Cleaner::execute_normalized(const uint8_t* block, SizeType bytes, S
             scale = m_scale2.as<float>();
         }
         const SizeType last = (d.nwin - 1) * m_n;
-        FB_CUDA(cudaMemcpyAsync(m_tail_loc.get(), m_loc.as<float>() + last, m_n * sizeof(float),
-                                cudaMemcpyDeviceToDevice, s));
-        FB_CUDA(cudaMemcpyAsync(m_tail_scale.get(), m_scale.as<float>() + last, m_n * sizeof(float),
-                                cudaMemcpyDeviceToDevice, s));
-        FB_CUDA(cudaMemcpyAsync(m_tail_out_loc.get(), loc + last, m_n * sizeof(float),
-                                cudaMemcpyDeviceToDevice, s));
-        FB_CUDA(cudaMemcpyAsync(m_tail_out_scale.get(), scale + last, m_n * sizeof(float),
-                                cudaMemcpyDeviceToDevice, s));
+        launch_keep_tail(m_n, m_loc.as<float>() + last, m_scale.as<float>() + last, loc + last, scale + last,
+                         m_tail_loc.as<float>(), m_tail_scale.as<float>(), m_tail_out_loc.as<float>(),
+                         m_tail_out_scale.as<float>(), s);
     }
     launch_normalize(d, m_work.as<float>(), loc, scale, m_mask_d.as<uint8_t>(), flip, capacity,
                      m_out.as<float>(), s);
@@ -690,11 +685,11 @@ void Cleaner::run_full(const Dims& d, cudaStream_t s) {
     const bool kchan   = c.kadane_channel_enabled != 0;
     const bool kspec   = c.kadane_spectrum_enabled != 0;
     auto* counters     = m_counters.as<unsigned long long>();
-    FB_CUDA(cudaMemsetAsync(counters, 0, kRepSlots * sizeof(unsigned long long), s));
+    launch_begin(d, counters, kRepSlots, m_unmeasured.as<uint32_t>(), m_kchan_any_d.as<uint8_t>(),
+                 m_time_flags_d.as<uint8_t>(), m_row_kchan.as<uint8_t>(), m_nslow.as<unsigned int>(), s);
 
     // ---- bandpass ----
     FB_CUDA(cudaEventRecord(m_ev[0], s));
-    FB_CUDA(cudaMemsetAsync(m_unmeasured.get(), 0, n * sizeof(uint32_t), s));
     launch_sample_rows(d, raw, m_samples.as<float>(), s);
     launch_bandpass(d, m_samples.as<float>(), m_loc.as<float>(), m_scale.as<float>(),
                     m_inv.as<float>(), m_unmeasured.as<uint32_t>(), s);

@@ -1305,7 +1305,6 @@ void decide_flags(const FlagParams& p, const FlagScratch& w, const uint64_t* goo
     const unsigned gt = grid_for(T, 256);
     k_dead<<<grid_for(n, 128), 128, 0, s>>>(n, p.nwin, good_prefix, unmeasured, lo, hi, mask, counters);
     FB_DECIDE_LAUNCH();
-    FB_CUDA(cudaMemsetAsync(time_flags, 0, std::max<uint64_t>(T, 1), s));
     if (T > 0) {
         if (p.broad)
             broadband(p, w, s_det, good_prefix, time_flags, counters, s);
@@ -1329,8 +1328,6 @@ void decide_flags(const FlagParams& p, const FlagScratch& w, const uint64_t* goo
         k_kchan_accept<<<grid_for(n, 128), 128, 0, s>>>(n, p.kchan_min_len, p.kchan_threshold, kpos_best, kneg_best,
                                                         mask, good_prefix, kchan_pos, kchan_neg, kchan_any);
         FB_DECIDE_LAUNCH();
-    } else {
-        FB_CUDA(cudaMemsetAsync(kchan_any, 0, n, s));
     }
     k_flag_list<<<1, kBlock, 0, s>>>(T, n, time_flags, mask, flagged, counters);
     FB_DECIDE_LAUNCH();

@@ -138,7 +138,7 @@ struct FlagScratch {
  * zero-DM fit, the accepted Kadane-along-time segments and the list of
  * flagged samples (increasing; its length in counters[kRepFlagged]). Every
  * step is skipped when no channel is good (good_prefix[n] == 0), as frost
- * skips them. */
+ * skips them. time_flags and kchan_any come in as launch_begin's zeros. */
 void decide_flags(const FlagParams& p, const FlagScratch& w, const uint64_t* good_prefix,
                   const uint32_t* unmeasured, const float* lo, const float* hi, const float* s_det,
                   const float* row_std, const uint8_t* kspec_whole, const ZdotSums* zsum,

@@ -159,14 +159,76 @@ __device__ __forceinline__ uint64_t draw(const ApplyParams& p, uint64_t stream, 
 
 // ---- finite check ---------------------------------------------------------
 
-__global__ void k_check_finite(const uint32_t* __restrict__ w, uint64_t n,
-                               unsigned long long* first_bad) {
+// Four 16-byte loads in flight a thread (1024 channels x 65 536: one word a
+// thread in turn took 119 us, 65 so); the first `head` words lead up to a
+// 16-byte boundary.
+__global__ void __launch_bounds__(256)
+    k_check_finite(const uint32_t* __restrict__ w, uint64_t n, uint64_t head, unsigned long long* first_bad) {
+    const uint64_t id     = blockIdx.x * static_cast<uint64_t>(blockDim.x) + threadIdx.x;
     const uint64_t stride = static_cast<uint64_t>(gridDim.x) * blockDim.x;
-    for (uint64_t i = blockIdx.x * static_cast<uint64_t>(blockDim.x) + threadIdx.x; i < n;
-         i += stride) {
-        if ((w[i] & 0x7F800000U) == 0x7F800000U)
+    auto test             = [&](uint32_t x, uint64_t i) {
+        if ((x & 0x7F800000U) == 0x7F800000U)
             atomicMin(first_bad, static_cast<unsigned long long>(i));
+    };
+    const uint64_t vecs = (n - head) / 4;
+    const uint4* v      = reinterpret_cast<const uint4*>(w + head);
+    for (uint64_t i = id; i < vecs; i += 4 * stride) {
+        uint4 x[4];
+#pragma unroll
+        for (int k = 0; k < 4; ++k)
+            x[k] = i + k * stride < vecs ? v[i + k * stride] : make_uint4(0, 0, 0, 0);
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            const uint64_t at = head + 4 * (i + k * stride);
+            test(x[k].x, at);
+            test(x[k].y, at + 1);
+            test(x[k].z, at + 2);
+            test(x[k].w, at + 3);
+        }
     }
+    const uint64_t tail = head + 4 * vecs;
+    if (id < head)
+        test(w[id], id);
+    if (id < n - tail)
+        test(w[tail + id], tail + id);
+}
+
+// ---- a gulp's start and end ---------------------------------------------------
+
+// Everything a cleaning pass counts or marks from zero, in one launch (six
+// memsets of a few KB took 3 us each).
+__global__ void __launch_bounds__(256)
+    k_begin(unsigned long long* __restrict__ counters, uint64_t nslots, uint32_t* __restrict__ unmeasured,
+            uint8_t* __restrict__ kchan_any, uint64_t nchans, uint8_t* __restrict__ time_flags,
+            uint8_t* __restrict__ row_kchan, uint64_t nsamps, unsigned int* __restrict__ nslow) {
+    const uint64_t stride = static_cast<uint64_t>(gridDim.x) * blockDim.x;
+    const uint64_t id     = blockIdx.x * static_cast<uint64_t>(blockDim.x) + threadIdx.x;
+    if (id < nslots)
+        counters[id] = 0;
+    if (id == 0)
+        *nslow = 0;
+    for (uint64_t i = id; i < nchans; i += stride) {
+        unmeasured[i] = 0;
+        kchan_any[i]  = 0;
+    }
+    for (uint64_t i = id; i < nsamps; i += stride) {
+        time_flags[i] = 0;
+        row_kchan[i]  = 0;
+    }
+}
+
+// The last window's constants, kept for short tails.
+__global__ void __launch_bounds__(256)
+    k_keep_tail(uint64_t nchans, const float* __restrict__ loc, const float* __restrict__ scale,
+                const float* __restrict__ out_loc, const float* __restrict__ out_scale, float* __restrict__ tail_loc,
+                float* __restrict__ tail_scale, float* __restrict__ tail_out_loc, float* __restrict__ tail_out_scale) {
+    const uint64_t c = blockIdx.x * static_cast<uint64_t>(blockDim.x) + threadIdx.x;
+    if (c >= nchans)
+        return;
+    tail_loc[c]       = loc[c];
+    tail_scale[c]     = scale[c];
+    tail_out_loc[c]   = out_loc[c];
+    tail_out_scale[c] = out_scale[c];
 }
 
 // ---- bandpass -------------------------------------------------------------
@@ -1986,8 +2048,28 @@ void launch_check_finite(const uint8_t* raw, uint64_t nwords, unsigned long long
                          cudaStream_t s) {
     if (nwords == 0)
         return;
-    const unsigned blocks = static_cast<unsigned>(std::min<uint64_t>((nwords + 255) / 256, 148 * 16));
-    k_check_finite<<<blocks, 256, 0, s>>>(reinterpret_cast<const uint32_t*>(raw), nwords, first_bad);
+    const uint64_t head   = std::min<uint64_t>(nwords, (16 - reinterpret_cast<uintptr_t>(raw) % 16) % 16 / 4);
+    const unsigned blocks = static_cast<unsigned>(std::min<uint64_t>((nwords + 4095) / 4096, 148 * 8));
+    k_check_finite<<<blocks, 256, 0, s>>>(reinterpret_cast<const uint32_t*>(raw), nwords, head, first_bad);
+    FB_COUNT_LAUNCH();
+}
+
+void launch_begin(const Dims& d, unsigned long long* counters, uint64_t nslots, uint32_t* unmeasured,
+                  uint8_t* kchan_any, uint8_t* time_flags, uint8_t* row_kchan, unsigned int* nslow, cudaStream_t s) {
+    const uint64_t most   = std::max({nslots, d.nchans, d.nsamps, uint64_t{1}});
+    const unsigned blocks = static_cast<unsigned>(std::min<uint64_t>((most + 255) / 256, 148 * 4));
+    k_begin<<<blocks, 256, 0, s>>>(counters, nslots, unmeasured, kchan_any, d.nchans, time_flags, row_kchan, d.nsamps,
+                                   nslow);
+    FB_COUNT_LAUNCH();
+}
+
+void launch_keep_tail(uint64_t nchans, const float* loc, const float* scale, const float* out_loc,
+                      const float* out_scale, float* tail_loc, float* tail_scale, float* tail_out_loc,
+                      float* tail_out_scale, cudaStream_t s) {
+    if (nchans == 0)
+        return;
+    k_keep_tail<<<grid1(nchans, 256), 256, 0, s>>>(nchans, loc, scale, out_loc, out_scale, tail_loc, tail_scale,
+                                                   tail_out_loc, tail_out_scale);
     FB_COUNT_LAUNCH();
 }
 
@@ -2139,7 +2221,6 @@ __global__ void __launch_bounds__(256)
 
 void launch_kchan_rows(const Dims& d, const Segment* kchan_pos, const Segment* kchan_neg,
                        const uint8_t* kchan_any, uint8_t* row_kchan, cudaStream_t s) {
-    FB_CUDA(cudaMemsetAsync(row_kchan, 0, d.nsamps, s));
     if (d.nsamps == 0 || d.nchans == 0)
         return;
     k_kchan_rows<<<static_cast<unsigned>(2 * d.nchans), 256, 0, s>>>(d.nchans, d.nsamps, kchan_pos, kchan_neg,
@@ -2161,7 +2242,6 @@ void launch_apply_unflagged(const Dims& d, const ApplyParams& p, const uint8_t* 
         return;
     if (d.nchans >= (uint64_t{1} << 31) || d.nsamps >= (uint64_t{1} << 31))
         throw Error(FROST_ERR_INVALID_ARGUMENT, "apply: too many channels or samples for one block");
-    FB_CUDA(cudaMemsetAsync(nslow, 0, sizeof(unsigned int), s));
     // 4-channel vectors need nchans % 4 == 0 and, for the byte loads of the
     // raw row, a 4-byte aligned block
     const bool vec = d.nchans % 4 == 0 && reinterpret_cast<uintptr_t>(raw) % 4 == 0;

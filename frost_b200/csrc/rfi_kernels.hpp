@@ -61,6 +61,18 @@ enum { kCountNarrow = 0, kCountKspec = 1, kCountKchan = 2, kCountFallback = 3, k
 void launch_check_finite(const uint8_t* raw, uint64_t nwords, unsigned long long* first_bad,
                          cudaStream_t s);
 
+/** A cleaning pass's zeros: report counters, unmeasured windows and Kadane
+ * marks of each channel, flags and Kadane marks of each sample, the listed
+ * rows' count. Queued before every other kernel of the pass. */
+void launch_begin(const Dims& d, unsigned long long* counters, uint64_t nslots, uint32_t* unmeasured,
+                  uint8_t* kchan_any, uint8_t* time_flags, uint8_t* row_kchan, unsigned int* nslow, cudaStream_t s);
+
+/** The constants of one window (`out_*`: after a transform), kept for short
+ * tails. */
+void launch_keep_tail(uint64_t nchans, const float* loc, const float* scale, const float* out_loc,
+                      const float* out_scale, float* tail_loc, float* tail_scale, float* tail_out_loc,
+                      float* tail_out_scale, cudaStream_t s);
+
 // Gathers the evenly spaced bandpass rows of every window into
 // samples[nwin][kMaxBandpassRows][nchans] as float.
 void launch_sample_rows(const Dims& d, const uint8_t* raw, float* samples, cudaStream_t s);
@@ -94,7 +106,7 @@ void launch_scan_cols(const Dims& d, const uint8_t* raw, const float* loc, const
                       Run* kpos_best, Run* kneg_best, cudaStream_t s);
 
 // row_kchan[t] = 1 for the rows some channel's Kadane-along-time segment
-// covers, else 0.
+// covers (launch_begin has set them all to 0).
 void launch_kchan_rows(const Dims& d, const Segment* kchan_pos, const Segment* kchan_neg,
                        const uint8_t* kchan_any, uint8_t* row_kchan, cudaStream_t s);
 
@@ -103,7 +115,7 @@ void launch_kchan_rows(const Dims& d, const Segment* kchan_pos, const Segment* k
 // their segments); a row with no clipped cell (row_clip), no segment
 // (row_kchan) and no span across frequency writes its clean values
 // without classifying its cells, the others are listed in slow_rows
-// (*nslow of them; nsamps entries of room) and cleaned cell by cell.
+// (*nslow of them, from launch_begin's 0; nsamps entries of room) and cleaned cell by cell.
 void launch_apply_unflagged(const Dims& d, const ApplyParams& p, const uint8_t* raw,
                             const float* loc, const float* scale, const float* inv,
                             const uint8_t* mask, const uint8_t* time_flags, const Span32* kspec_pos,
