@@ -918,35 +918,42 @@ void launch_level2(const FusedOp* ops, int64_t nrows, LevelView in, LevelView ou
 }
 
 namespace {
-// dst[r][0 .. w) = src[r][0 .. w) in 16-byte vectors, w vectors a row.
+// The last need[r] columns of each row's history, a warp a row: dst[r] and
+// src[r] are rows of w 16-byte vectors (ES-byte columns), of which a row that
+// no later step reads shifted needs none, one that is searched the widest
+// boxcar less one, and the others their largest shift. Copying every row's
+// whole history took 2.43 of 30 ms at 4096 channels x 65 536, fp32 (the top
+// levels' rows are 17 000 columns and only the upper half-band's are read,
+// half of those columns on average), these copies 0.48. With SHIFT the source rows
+// start at any even byte (a ragged gulp's last columns): the vectors are put
+// together from aligned words, read only where they hold bytes of the row.
+template <int ES, bool SHIFT>
 __global__ void __launch_bounds__(256)
-    k_copy_rows16(uint4* __restrict__ dst, int64_t dpitch, const uint4* __restrict__ src, int64_t spitch,
-                  uint32_t w, uint32_t n) {
-    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        const uint32_t r = i / w, c = i - r * w;
-        dst[r * dpitch + c] = src[r * spitch + c];
-    }
-}
-
-// The same from rows that start at any even byte (a ragged gulp's last
-// columns): the destination's 16-byte vectors put together from aligned
-// words, shifted by two bytes where a row starts inside one. Words are read
-// only where they hold bytes of the row.
-__global__ void __launch_bounds__(256)
-    k_copy_rows_shifted(uint4* __restrict__ dst, int64_t dpitch, const unsigned char* __restrict__ src,
-                        int64_t spitch, uint32_t w, uint32_t n) {
-    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        const uint32_t r = i / w, c = i - r * w;
-        const unsigned char* a = src + r * spitch + c * 16;
-        const uint32_t m       = static_cast<uint32_t>(reinterpret_cast<uintptr_t>(a) & 3U);
-        const uint32_t* v      = reinterpret_cast<const uint32_t*>(a - m);
-        uint32_t x[5];
+    k_copy_history(uint4* __restrict__ dst, int64_t dpitch, const unsigned char* __restrict__ src, int64_t spitch,
+                   int32_t w, const int32_t* __restrict__ need, int64_t rows) {
+    const int lane      = threadIdx.x & 31;
+    const int64_t warps = static_cast<int64_t>(gridDim.x) * (blockDim.x / 32);
+    for (int64_t r = static_cast<int64_t>(blockIdx.x) * (blockDim.x / 32) + (threadIdx.x >> 5); r < rows; r += warps) {
+        const int32_t n = need[r] * ES / 16;
+#pragma unroll 4
+        for (int32_t c = w - n + lane; c < w; c += 32) {
+            const unsigned char* a = src + r * spitch + static_cast<int64_t>(c) * 16;
+            uint4 v;
+            if constexpr (SHIFT) {
+                const uint32_t m  = static_cast<uint32_t>(reinterpret_cast<uintptr_t>(a) & 3U);
+                const uint32_t* p = reinterpret_cast<const uint32_t*>(a - m);
+                uint32_t x[5];
 #pragma unroll
-        for (int k = 0; k < 4; ++k)
-            x[k] = v[k];
-        x[4] = m != 0 ? v[4] : 0U;
-        dst[r * dpitch + c] = make_uint4(__funnelshift_r(x[0], x[1], 8 * m), __funnelshift_r(x[1], x[2], 8 * m),
-                                         __funnelshift_r(x[2], x[3], 8 * m), __funnelshift_r(x[3], x[4], 8 * m));
+                for (int k = 0; k < 4; ++k)
+                    x[k] = p[k];
+                x[4] = m != 0 ? p[4] : 0U;
+                v    = make_uint4(__funnelshift_r(x[0], x[1], 8 * m), __funnelshift_r(x[1], x[2], 8 * m),
+                                  __funnelshift_r(x[2], x[3], 8 * m), __funnelshift_r(x[3], x[4], 8 * m));
+            } else {
+                v = *reinterpret_cast<const uint4*>(a);
+            }
+            dst[r * dpitch + c] = v;
+        }
     }
 }
 
@@ -983,46 +990,43 @@ void copy_floats(float* dst, size_t dpitch, const float* src, size_t spitch, siz
 }
 } // namespace
 
-// A ragged gulp's rows are copied by a kernel too: a 2-D memcpy of them took
-// 0.32 of the 4.0 ms of a 1000-channel search of 50 001 samples (3.75 now).
-void copy_rows(void* dst, size_t dpitch, const void* src, size_t spitch, size_t width, size_t rows,
-               cudaStream_t s) {
-    if (rows == 0 || width == 0)
-        return;
-    const uintptr_t to   = reinterpret_cast<uintptr_t>(dst) | dpitch | width;
-    const uintptr_t from = reinterpret_cast<uintptr_t>(src) | spitch;
-    const size_t n       = rows * (width / 16);
-    if (to % 16 != 0 || from % 2 != 0 || n > 0x7FFFFFFFU) {
-        FB_CUDA(cudaMemcpy2DAsync(dst, dpitch, src, spitch, width, rows, cudaMemcpyDeviceToDevice, s));
-        return;
-    }
-    if (from % 16 != 0)
-        k_copy_rows_shifted<<<copy_blocks(n), 256, 0, s>>>(
-            static_cast<uint4*>(dst), static_cast<int64_t>(dpitch / 16), static_cast<const unsigned char*>(src),
-            static_cast<int64_t>(spitch), static_cast<uint32_t>(width / 16), static_cast<uint32_t>(n));
-    else
-        k_copy_rows16<<<copy_blocks(n), 256, 0, s>>>(
-            static_cast<uint4*>(dst), static_cast<int64_t>(dpitch / 16), static_cast<const uint4*>(src),
-            static_cast<int64_t>(spitch / 16), static_cast<uint32_t>(width / 16), static_cast<uint32_t>(n));
+namespace {
+// Byte pitches and width; the destination rows and the width are multiples of
+// 16 bytes (histories are whole vectors of columns).
+void copy_history(void* dst, int64_t dpitch, const void* src, int64_t spitch, int64_t width, int es,
+                  const int32_t* need, int64_t rows, cudaStream_t s) {
+    const uintptr_t to   = reinterpret_cast<uintptr_t>(dst) | static_cast<uintptr_t>(dpitch | width);
+    const uintptr_t from = reinterpret_cast<uintptr_t>(src) | static_cast<uintptr_t>(spitch);
+    if (to % 16 != 0 || from % 2 != 0)
+        throw Error(FROST_ERR_INTERNAL, "history: rows are not whole vectors");
+    const bool shift = from % 16 != 0;
+    const auto k     = es == 2 ? (shift ? &k_copy_history<2, true> : &k_copy_history<2, false>)
+                               : (shift ? &k_copy_history<4, true> : &k_copy_history<4, false>);
+    k<<<copy_blocks(static_cast<size_t>(rows) * 32), 256, 0, s>>>(
+        static_cast<uint4*>(dst), dpitch / 16, static_cast<const unsigned char*>(src), spitch,
+        static_cast<int32_t>(width / 16), need, rows);
     FB_LAUNCH_CHECK();
 }
+} // namespace
 
-void launch_save_history(LevelView v, int64_t rows, int32_t hist, int32_t n_valid, void* hist_buf,
-                         cudaStream_t s) {
+void launch_save_history(LevelView v, int64_t rows, int32_t hist, const int32_t* need, int32_t n_valid,
+                         void* hist_buf, cudaStream_t s) {
     if (rows == 0 || hist == 0)
         return;
-    const size_t es  = v.fp16 ? 2 : 4;
-    const char* src  = static_cast<const char*>(v.data) + (v.base + n_valid - hist) * es;
-    copy_rows(hist_buf, hist * es, src, v.pitch * es, hist * es, static_cast<size_t>(rows), s);
+    const int es    = v.fp16 ? 2 : 4;
+    const char* src = static_cast<const char*>(v.data) + static_cast<int64_t>(v.base + n_valid - hist) * es;
+    copy_history(hist_buf, static_cast<int64_t>(hist) * es, src, v.pitch * es, static_cast<int64_t>(hist) * es, es,
+                 need, rows, s);
 }
 
-void launch_load_history(LevelView v, int64_t rows, int32_t hist, const void* hist_buf,
+void launch_load_history(LevelView v, int64_t rows, int32_t hist, const int32_t* need, const void* hist_buf,
                          cudaStream_t s) {
     if (rows == 0 || hist == 0)
         return;
-    const size_t es = v.fp16 ? 2 : 4;
-    char* dst       = static_cast<char*>(v.data) + (v.base - hist) * es;
-    copy_rows(dst, v.pitch * es, hist_buf, hist * es, hist * es, static_cast<size_t>(rows), s);
+    const int es = v.fp16 ? 2 : 4;
+    char* dst    = static_cast<char*>(v.data) + static_cast<int64_t>(v.base - hist) * es;
+    copy_history(dst, v.pitch * es, hist_buf, static_cast<int64_t>(hist) * es, static_cast<int64_t>(hist) * es, es,
+                 need, rows, s);
 }
 
 void launch_save_input_history(const float* wf, int64_t pitch, int64_t t0, int32_t n_valid,

@@ -97,19 +97,15 @@ void launch_level2(const FusedOp* ops, int64_t nrows, LevelView in, LevelView ou
 void launch_level_segs(LevelSeg* segs, int n, bool fused, bool fp16, int32_t stages, cudaStream_t s,
                        int32_t ctas = 0, long long wait_limit = kDefaultWaitLimit);
 
-/** dst[r][0 .. width) = src[r][0 .. width) for `rows` rows of pitches
- * dpitch / spitch bytes (device memory): 16-byte vectors when pointers,
- * pitches and width allow, cudaMemcpy2DAsync otherwise. */
-void copy_rows(void* dst, size_t dpitch, const void* src, size_t spitch, size_t width, size_t rows,
-               cudaStream_t s);
-
-/** Copies the last `hist` columns ending at column base + n_valid of every
- * row of `view` into hist_buf[rows][hist]. */
-void launch_save_history(LevelView view, int64_t rows, int32_t hist, int32_t n_valid,
+/** Copies the last need[r] (<= hist, both multiples of 8) columns ending at
+ * column base + n_valid of every row r of `view` into the end of
+ * hist_buf[r][hist]. */
+void launch_save_history(LevelView view, int64_t rows, int32_t hist, const int32_t* need, int32_t n_valid,
                          void* hist_buf, cudaStream_t s);
 
-/** Copies hist_buf[rows][hist] into columns [base - hist, base). */
-void launch_load_history(LevelView view, int64_t rows, int32_t hist, const void* hist_buf,
+/** Copies those columns of hist_buf[rows][hist] into columns [base - need[r],
+ * base). */
+void launch_load_history(LevelView view, int64_t rows, int32_t hist, const int32_t* need, const void* hist_buf,
                          cudaStream_t s);
 
 /** Copies level rows `rows[0..nrows)` (tile columns [0, n_valid)) to

@@ -350,8 +350,11 @@ Engine::Footprint Engine::estimate(const frost_dedisp_plan_config& dd, const fro
         hist  = std::max(hist, h_bytes);
         fused = std::max<SizeType>(fused, sc.fused.size() * sizeof(FusedOp));
     }
+    SizeType rows_all = 0;
+    for (int h = 1; h <= L; ++h)
+        rows_all += static_cast<SizeType>(plan.level_rows(h));
     const SizeType in_hist = b16(static_cast<SizeType>(C) * plan.level_history(0) * sizeof(float));
-    f.table_bytes += fused;
+    f.table_bytes += fused + b16(rows_all * sizeof(int32_t));
     f.level_bytes     = buf[0] + buf[1];
     f.history_bytes   = hist + 2 * in_hist;
     f.transient_bytes = static_cast<SizeType>(C) * std::min<SizeType>(dd.block_nsamps, 4096) * sizeof(float);
@@ -369,6 +372,15 @@ Engine::Schedule Engine::make_schedule(const Plan& plan, const std::vector<int64
         keep[p.height] = 1;
     Schedule sc;
     sc.buf_of.assign(L + 1, -1);
+    sc.need_off.assign(L + 2, 0);
+    for (int h = 1; h <= L; ++h)
+        sc.need_off[h + 1] = sc.need_off[h] + plan.level_rows(h);
+    sc.need.assign(static_cast<size_t>(sc.need_off[L + 1]), 0);
+    auto reads = [&](int h, int64_t row, int32_t columns) {
+        int32_t& n      = sc.need[static_cast<size_t>(sc.need_off[h] + row)];
+        n               = std::max(n, columns);
+        sc.hist_len[h]  = std::max(sc.hist_len[h], columns);
+    };
     sc.hist_len.assign(L + 1, 0);
     sc.hist_len[0] = plan.level_history(0);
     sc.steps.push_back({1, 0, false, 0});
@@ -390,7 +402,7 @@ Engine::Schedule Engine::make_schedule(const Plan& plan, const std::vector<int64
                 }
                 for (int j = 1; j < 4; ++j)
                     if (f.row[j] >= 0)
-                        sc.hist_len[h] = std::max(sc.hist_len[h], f.shift[j]);
+                        reads(h, f.row[j], f.shift[j]);
                 sc.fused.push_back(f);
             }
             h += 2;
@@ -398,18 +410,23 @@ Engine::Schedule Engine::make_schedule(const Plan& plan, const std::vector<int64
             st = {h + 1, h, false, row_op_offset[h + 1]};
             for (const RowOp& op : plan.row_ops(h + 1))
                 if (op.hi_row >= 0)
-                    sc.hist_len[h] = std::max(sc.hist_len[h], op.shift);
+                    reads(h, op.hi_row, op.shift);
             h += 1;
         }
         sc.buf_of[st.out] = static_cast<int>(sc.steps.size() % 2);
         sc.steps.push_back(st);
     }
-    for (const auto& p : plan_planes)
+    for (const auto& p : plan_planes) {
         sc.hist_len[p.height] = std::max(sc.hist_len[p.height], plan.widths().back() - 1);
+        for (const auto r : p.level_row)
+            reads(p.height, r, plan.widths().back() - 1);
+    }
     // whole 16-byte vectors of fp16 (and fp32) columns, so that the history
     // copies move aligned vectors (a longer history is a superset)
     for (int h = 1; h <= L; ++h)
         sc.hist_len[h] = static_cast<int32_t>(round_up(sc.hist_len[h], 8));
+    for (int32_t& n : sc.need)
+        n = static_cast<int32_t>(round_up(n, 8));
     return sc;
 }
 
@@ -418,6 +435,8 @@ void Engine::build_schedule(bool fuse) {
     m_steps     = std::move(sc.steps);
     m_buf_of    = std::move(sc.buf_of);
     m_hist_len  = std::move(sc.hist_len);
+    m_need_off  = std::move(sc.need_off);
+    upload(m_hist_need, sc.need, m_stream);
     upload(m_fused_ops, sc.fused, m_stream);
     m_fuse = fuse;
     if (m_graph != nullptr) {
@@ -685,7 +704,7 @@ int Engine::batch_mid(int64_t round, cudaStream_t s, RoundWork& w) {
     const int h           = st.out;
     const int32_t n_valid = static_cast<int32_t>(std::min<int64_t>(m_tile, static_cast<int64_t>(m_batch_nsamps) - t_off));
     const LevelView out   = view(h);
-    launch_load_history(out, m_plan.level_rows(h), m_hist_len[h], m_hist[h].get(), s);
+    launch_load_history(out, m_plan.level_rows(h), m_hist_len[h], hist_need(h), m_hist[h].get(), s);
     if (m_height_g1[h] > m_height_g0[h]) {
         w.has_search   = true;
         w.chunk        = m_search_chunk;
@@ -710,13 +729,13 @@ int Engine::batch_post(int64_t round, cudaStream_t s) {
     const Step& st        = m_steps[si];
     int n                 = 0;
     if (si > 0) {
-        launch_save_history(view(st.in), m_plan.level_rows(st.in), m_hist_len[st.in], n_valid,
+        launch_save_history(view(st.in), m_plan.level_rows(st.in), m_hist_len[st.in], hist_need(st.in), n_valid,
                             m_hist[st.in].get(), s);
         ++n;
     }
     if (static_cast<int64_t>(si) == nsteps - 1) {
         const int L = m_plan.levels();
-        launch_save_history(view(L), m_plan.level_rows(L), m_hist_len[L], n_valid, m_hist[L].get(), s);
+        launch_save_history(view(L), m_plan.level_rows(L), m_hist_len[L], hist_need(L), n_valid, m_hist[L].get(), s);
         ++n;
     }
     return n;
@@ -890,7 +909,8 @@ SizeType Engine::device_bytes() const {
                                   &m_inv_or, &m_mask_d, &m_mask_or_d, &m_carry, &m_row_counts, &m_cands,
                                   &m_counters, &m_clock, &m_frontier, &m_capture_rows,
                                   &m_sort_keys[0], &m_sort_keys[1], &m_sort_vals[0], &m_sort_vals[1],
-                                  &m_sort_hist, &m_cands_sorted, &m_cand_range, &m_fs_ops, &m_fs_rows};
+                                  &m_sort_hist, &m_cands_sorted, &m_cand_range, &m_fs_ops, &m_fs_rows,
+                                  &m_hist_need};
     for (const auto* b : rest)
         total += b->bytes();
     for (const auto& b : m_capture)
@@ -1101,7 +1121,7 @@ void Engine::run_tiles(const float* wf, SizeType nsamps, cudaStream_t s) {
                     static_cast<uint64_t>(m_plan.level_rows(st.in) + m_plan.level_rows(h)) * m_ncols * es;
             }
             timed(kHistory, s, [&] {
-                launch_load_history(out, m_plan.level_rows(h), m_hist_len[h], m_hist[h].get(), s);
+                launch_load_history(out, m_plan.level_rows(h), m_hist_len[h], hist_need(h), m_hist[h].get(), s);
             });
             if (m_height_g1[h] > m_height_g0[h]) {
                 const bool fs   = si > 0 && fused_search(st);
@@ -1135,12 +1155,12 @@ void Engine::run_tiles(const float* wf, SizeType nsamps, cudaStream_t s) {
             }
             if (si > 0)
                 timed(kHistory, s, [&] {
-                    launch_save_history(view(st.in), m_plan.level_rows(st.in), m_hist_len[st.in],
+                    launch_save_history(view(st.in), m_plan.level_rows(st.in), m_hist_len[st.in], hist_need(st.in),
                                         n_valid, m_hist[st.in].get(), s);
                 });
         }
         timed(kHistory, s, [&] {
-            launch_save_history(view(L), m_plan.level_rows(L), m_hist_len[L], n_valid, m_hist[L].get(), s);
+            launch_save_history(view(L), m_plan.level_rows(L), m_hist_len[L], hist_need(L), n_valid, m_hist[L].get(), s);
         });
     }
 }

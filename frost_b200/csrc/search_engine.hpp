@@ -164,12 +164,17 @@ private:
         std::vector<Step> steps;
         std::vector<int> buf_of;
         std::vector<int32_t> hist_len;
+        std::vector<int32_t> need;     // per stored row: history columns that anything reads
+        std::vector<int64_t> need_off; // level -> its first row in `need`
         std::vector<FusedOp> fused;
     };
     /** The FDMT schedule of `plan` (host only): steps, the buffer of every
      * stored level, history lengths and the fused ops. */
     static Schedule make_schedule(const Plan& plan, const std::vector<int64_t>& row_op_offset, bool fuse);
     static void validate(const frost_dedisp_plan_config& dd, const frost_boxcar_config& bc, const Plan& plan);
+    std::vector<int64_t> m_need_off;
+    DeviceBuffer m_hist_need; // Schedule::need
+    const int32_t* hist_need(int h) const { return m_hist_need.as<int32_t>() + m_need_off[h]; }
     DeviceBuffer m_fused_ops;
     bool m_fuse        = true; // fused two-level steps in the schedule
     int32_t m_level_tpc = 16;  // tiles of 2048 columns per level-kernel CTA

@@ -8,7 +8,7 @@ FP64 oracle with the search tests' criteria."""
 import numpy as np
 import pytest
 
-from frost_b200.config import BoxcarConfig, PeakMode
+from frost_b200.config import BoxcarConfig, PeakMode, Storage
 from tests.search_cases import compare, make_stream, plan_config, run_engine
 from tests.test_search_gpu import PULSES, oracle_for
 
@@ -38,3 +38,23 @@ def test_bounds_match_the_oracle(gulp, max_boxcar, wtsp, trapezoid, mode, thresh
     ref = oracle_for(pc, bc).search(masked, gulp, masks)
     n, missing, extra, bad = compare(cands, ref, bc.detect_thresh)
     assert n > 0 and not missing and not extra and not bad, (missing[:3], extra[:3], bad[:3])
+
+
+@pytest.mark.parametrize("storage", [Storage.FP32, Storage.FP16])
+@pytest.mark.parametrize("gulp,tile,depth", [(3001, 0, 0), (5003, 4096, 2), (8200, 0, 1)])
+def test_histories_of_ragged_gulps(gulp, tile, depth, storage):
+    """Every row keeps the columns its readers shift into, for gulps that end
+    at any column: the third gulp's planes against the oracle's rows over the
+    whole stream (the storage precisions' bounds of the search tests)."""
+    from frost_b200.search import FDMTBoxcar
+    pc = plan_config(nchans=50, depth=depth, gulp=gulp, dm_max=45.0)
+    bc = BoxcarConfig(max_boxcar=40, detect_thresh=8.0, storage=storage, max_candidates=1 << 18)
+    stream = make_stream(pc, 3, seed=gulp, pulses=PULSES)
+    eng = FDMTBoxcar(pc, bc, tile_nsamps=tile)
+    eng.capture_planes(True)
+    run_engine(eng, stream, gulp, drain=False)
+    bound = 1e-5 if storage == Storage.FP32 else 1e-2
+    for p, band in enumerate(oracle_for(pc, bc).bands):
+        rows = oracle_for(pc, bc).dedisperse(stream, band)[:, -gulp:]
+        rms = np.sqrt(np.mean(rows ** 2, axis=1, keepdims=True)) + 1e-12
+        assert np.max(np.abs(eng.plane_data(p, gulp) - rows) / rms) < bound, p
