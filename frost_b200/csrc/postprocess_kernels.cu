@@ -14,6 +14,7 @@
 // Built with --fmad=false: the predicates of pp_math.cuh must round like
 // the reference's strict-IEEE host code.
 
+#include <algorithm>
 #include <atomic>
 #include <utility>
 
@@ -123,48 +124,6 @@ __global__ void k_rs_hist(const u64* __restrict__ keys, size_t n, int shift, u32
     }
     __syncthreads();
     hist[static_cast<size_t>(threadIdx.x) * nblk + blockIdx.x] = h[threadIdx.x];
-}
-
-/** In-place exclusive scan of a[0, total) by one block of 1024 threads;
- * *sum = the total when sum is given. */
-__global__ void k_scan_single(u32* __restrict__ a, size_t total, u32* sum) {
-    __shared__ u32 ws[32];
-    const size_t per = (total + blockDim.x - 1) / blockDim.x;
-    const size_t b   = threadIdx.x * per;
-    const size_t e   = b + per < total ? b + per : total;
-    u32 s            = 0;
-    for (size_t i = b; i < e; ++i)
-        s += a[i];
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    u32 x          = s;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-        const u32 y = __shfl_up_sync(0xffffffffu, x, o);
-        if (lane >= o)
-            x += y;
-    }
-    if (lane == 31)
-        ws[w] = x;
-    __syncthreads();
-    if (w == 0) {
-        u32 v = lane < static_cast<int>(blockDim.x >> 5) ? ws[lane] : 0u;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const u32 y = __shfl_up_sync(0xffffffffu, v, o);
-            if (lane >= o)
-                v += y;
-        }
-        ws[lane] = v;
-    }
-    __syncthreads();
-    u32 run = x - s + (w > 0 ? ws[w - 1] : 0u);
-    for (size_t i = b; i < e; ++i) {
-        const u32 v = a[i];
-        a[i]        = run;
-        run += v;
-    }
-    if (sum != nullptr && threadIdx.x == blockDim.x - 1)
-        *sum = ws[(blockDim.x >> 5) - 1];
 }
 
 /** Stable scatter of one 8-bit digit: items of a tile keep their order
@@ -323,11 +282,11 @@ __global__ void __launch_bounds__(1024)
     }
 }
 
-/** Exclusive scan of in[0, n) by one block of 1024 threads, 4096 a round;
- * *sum = the total. */
+/** Exclusive scan of in[0, n) into out (in itself, too) by one block of 1024
+ * threads, 4096 words a round; *sum, when given, is the total. */
 constexpr size_t kSmallScan = 32768;
 __global__ void __launch_bounds__(1024)
-    k_scan_small(const u32* __restrict__ in, u32* __restrict__ out, u32 n, u32* __restrict__ sum) {
+    k_scan_small(const u32* in, u32* out, u32 n, u32* sum) {
     __shared__ u32 ws[32];
     const int t = threadIdx.x, lane = t & 31, w = t >> 5;
     u32 carry = 0;
@@ -370,7 +329,7 @@ __global__ void __launch_bounds__(1024)
         }
         __syncthreads();
     }
-    if (t == 0)
+    if (t == 0 && sum != nullptr)
         *sum = carry;
 }
 
@@ -959,65 +918,71 @@ __global__ void k_ready_flags(size_t n, const u32* __restrict__ recent, int fina
 
 // ---- sub-band dedup ---------------------------------------------------------------------
 
+// All pairs of rows, a CTA for 128 rows i against `chunk` rows j: the tests
+// are chains of double divisions, bound by latency, and a CTA that took its
+// rows against all others left ten of them for 1300 rows (1131 us, 25 so).
+// A row's dm_step is worked out once.
 constexpr int kPairTile = 128;
 
-__global__ void __launch_bounds__(kPairTile) k_dedup_pairs(const frost_giant* __restrict__ rows, size_t n,
-                                                           frost_cluster_tolerances tol, float tsamp,
-                                                           u32* parent) {
-    __shared__ Pt tile[kPairTile];
-    volatile u32* p = parent;
-    const size_t i  = blockIdx.x * static_cast<size_t>(kPairTile) + threadIdx.x;
-    const Pt a      = i < n ? pt_of(rows[i]) : Pt{};
-    for (size_t j0 = blockIdx.x * static_cast<size_t>(kPairTile); j0 < n; j0 += kPairTile) {
-        const size_t jl = j0 + threadIdx.x;
-        if (jl < n)
-            tile[threadIdx.x] = pt_of(rows[jl]);
-        __syncthreads();
-        if (i < n) {
-            const size_t m = (n - j0) < static_cast<size_t>(kPairTile) ? n - j0 : kPairTile;
-            for (size_t jj = 0; jj < m; ++jj) {
-                const size_t j = j0 + jj;
-                if (j > i && on_same_curve(a, tile[jj], tol, tsamp))
-                    unite(p, static_cast<u32>(i), static_cast<u32>(j));
-            }
+/** Rows j0 .. j0 + m of `rows` (through `order` when given) with their steps. */
+struct PairTile {
+    Pt pt[kPairTile];
+    double step[kPairTile];
+    __device__ __forceinline__ void load(const frost_giant* __restrict__ rows, const u32* __restrict__ order,
+                                         size_t j0, size_t m, float tsamp) {
+        if (threadIdx.x < m) {
+            pt[threadIdx.x]   = pt_of(rows[order != nullptr ? order[j0 + threadIdx.x] : j0 + threadIdx.x]);
+            step[threadIdx.x] = dm_step(pt[threadIdx.x].flo, pt[threadIdx.x].fhi, tsamp);
         }
+        __syncthreads();
+    }
+};
+
+__global__ void __launch_bounds__(kPairTile) k_dedup_pairs(const frost_giant* __restrict__ rows, size_t n,
+                                                           frost_cluster_tolerances tol, float tsamp, u32 chunk,
+                                                           u32* parent) {
+    __shared__ PairTile tile;
+    const size_t i0   = blockIdx.x * static_cast<size_t>(kPairTile);
+    const size_t i    = i0 + threadIdx.x;
+    const Pt a        = i < n ? pt_of(rows[i]) : Pt{};
+    const double step = dm_step(a.flo, a.fhi, tsamp);
+    volatile u32* p   = parent;
+    for (size_t j0 = blockIdx.y * static_cast<size_t>(chunk); j0 < n; j0 += static_cast<size_t>(gridDim.y) * chunk) {
+        const size_t m = n - j0 < chunk ? n - j0 : chunk;
+        if (j0 + m <= i0 + 1)
+            continue; // every j <= every i
+        tile.load(rows, nullptr, j0, m, tsamp);
+        if (i < n)
+            for (size_t jj = 0; jj < m; ++jj)
+                if (j0 + jj > i && on_same_curve(a, tile.pt[jj], step, tile.step[jj], tol, tsamp))
+                    unite(p, static_cast<u32>(i), static_cast<u32>(j0 + jj));
         __syncthreads();
     }
 }
 
+// fm[k] (k on entry): the first m < k, both in `order`, that lies on k's
+// curve. Chunks of m race: each lowers fm[k] to its first match.
 __global__ void __launch_bounds__(kPairTile) k_first_match(const frost_giant* __restrict__ rows,
                                                            const u32* __restrict__ order, size_t n,
-                                                           frost_cluster_tolerances tol, float tsamp,
-                                                           u32* __restrict__ fm) {
-    __shared__ Pt tile[kPairTile];
-    const size_t k    = blockIdx.x * static_cast<size_t>(kPairTile) + threadIdx.x;
+                                                           frost_cluster_tolerances tol, float tsamp, u32 chunk,
+                                                           u32* fm) {
+    __shared__ PairTile tile;
+    const size_t k0   = blockIdx.x * static_cast<size_t>(kPairTile);
+    const size_t k    = k0 + threadIdx.x;
     const Pt b        = k < n ? pt_of(rows[order[k]]) : Pt{};
-    u32 found         = k < n ? static_cast<u32>(k) : 0u;
-    bool done         = k >= n;
-    const size_t kmax = (blockIdx.x + 1) * static_cast<size_t>(kPairTile) < n
-                            ? (blockIdx.x + 1) * static_cast<size_t>(kPairTile)
-                            : n;
-    for (size_t m0 = 0; m0 < kmax; m0 += kPairTile) {
-        const size_t ml = m0 + threadIdx.x;
-        if (ml < n)
-            tile[threadIdx.x] = pt_of(rows[order[ml]]);
-        __syncthreads();
-        if (!done) {
-            for (size_t mm = 0; mm < static_cast<size_t>(kPairTile); ++mm) {
-                const size_t m = m0 + mm;
-                if (m >= k)
-                    break;
-                if (on_same_curve(tile[mm], b, tol, tsamp)) {
-                    found = static_cast<u32>(m);
-                    done  = true;
+    const double step = dm_step(b.flo, b.fhi, tsamp);
+    for (size_t m0 = blockIdx.y * static_cast<size_t>(chunk); m0 < n && m0 < k0 + kPairTile - 1;
+         m0 += static_cast<size_t>(gridDim.y) * chunk) {
+        const size_t mn = n - m0 < chunk ? n - m0 : chunk;
+        tile.load(rows, order, m0, mn, tsamp);
+        if (k < n && *const_cast<volatile u32*>(fm + k) >= m0)
+            for (size_t mm = 0; mm < mn && m0 + mm < k; ++mm)
+                if (on_same_curve(tile.pt[mm], b, tile.step[mm], step, tol, tsamp)) {
+                    atomicMin(fm + k, static_cast<u32>(m0 + mm));
                     break;
                 }
-            }
-        }
         __syncthreads();
     }
-    if (k < n)
-        fm[k] = found;
 }
 
 __global__ void k_resolve_seeded(const u32* __restrict__ order, const u32* __restrict__ fm, size_t n,
@@ -1154,7 +1119,7 @@ void radix_sort(u64*& keys, u32*& vals, u64*& keys_alt, u32*& vals_alt, size_t n
     for (int shift = 0; shift < bits; shift += 8) {
         k_rs_hist<<<nblk, kThreads, 0, s>>>(keys, n, shift, hist, nblk);
         FB_LAUNCH_CHECK();
-        k_scan_single<<<1, 1024, 0, s>>>(hist, static_cast<size_t>(nblk) * 256, nullptr);
+        k_scan_small<<<1, 1024, 0, s>>>(hist, hist, nblk * 256, nullptr);
         FB_LAUNCH_CHECK();
         k_rs_scatter<<<nblk, kThreads, 0, s>>>(keys, vals, keys_alt, vals_alt, n, shift, hist, nblk);
         FB_LAUNCH_CHECK();
@@ -1198,7 +1163,7 @@ void exclusive_scan(const u32* in, u32* out, size_t n, u32* tile_sums, u32* tota
     const unsigned nt = static_cast<unsigned>((n + kTile - 1) / kTile);
     k_scan_tiles<<<nt, kThreads, 0, s>>>(in, n, out, tile_sums);
     FB_LAUNCH_CHECK();
-    k_scan_single<<<1, 1024, 0, s>>>(tile_sums, nt, total);
+    k_scan_small<<<1, 1024, 0, s>>>(tile_sums, tile_sums, nt, total);
     FB_LAUNCH_CHECK();
     count();
     count();
@@ -1419,11 +1384,19 @@ void launch_ready_flags(size_t n, const u32* recent, int final_call, u32* rflag,
     count();
 }
 
+// Rows j that a CTA of the pair kernels takes at a time: 16 while only their
+// number makes CTAs enough, a whole tile from there on.
+static u32 pair_chunk(size_t n) { return n <= 4096 ? 16 : kPairTile; }
+static dim3 pair_grid(size_t n, u32 chunk) {
+    return dim3(blocks_for(n, kPairTile), static_cast<unsigned>(std::min<size_t>((n + chunk - 1) / chunk, 65535)));
+}
+
 void launch_dedup_pairs(const frost_giant* rows, size_t n, const frost_cluster_tolerances& tol, float tsamp,
                         u32* parent, cudaStream_t s) {
     if (n < 2)
         return;
-    k_dedup_pairs<<<blocks_for(n, kPairTile), kPairTile, 0, s>>>(rows, n, tol, tsamp, parent);
+    const u32 chunk = pair_chunk(n);
+    k_dedup_pairs<<<pair_grid(n, chunk), kPairTile, 0, s>>>(rows, n, tol, tsamp, chunk, parent);
     FB_LAUNCH_CHECK();
     count();
 }
@@ -1432,7 +1405,9 @@ void launch_first_match(const frost_giant* rows, const u32* order, size_t n,
                         const frost_cluster_tolerances& tol, float tsamp, u32* fm, cudaStream_t s) {
     if (n == 0)
         return;
-    k_first_match<<<blocks_for(n, kPairTile), kPairTile, 0, s>>>(rows, order, n, tol, tsamp, fm);
+    launch_iota(fm, n, s);
+    const u32 chunk = pair_chunk(n);
+    k_first_match<<<pair_grid(n, chunk), kPairTile, 0, s>>>(rows, order, n, tol, tsamp, chunk, fm);
     FB_LAUNCH_CHECK();
     count();
 }

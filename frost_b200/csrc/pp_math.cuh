@@ -140,15 +140,17 @@ PP_HD bool dm_within_smear(const Pt& a, const Pt& b, const frost_cluster_toleran
     return delta <= (smear * delay * step);
 }
 
-/** on_same_curve(a, b, tol, tsamp) (subband_dedup.cpp:85-150). */
-PP_HD bool on_same_curve(const Pt& a, const Pt& b, const frost_cluster_tolerances& t, float tsamp) {
+/** on_same_curve(a, b, tol, tsamp) (subband_dedup.cpp:85-150), step_a and
+ * step_b the dm_step of each one's band. */
+PP_HD bool on_same_curve(const Pt& a, const Pt& b, double step_a, double step_b, const frost_cluster_tolerances& t,
+                         float tsamp) {
     const u64 sa = span_of(a.cb, a.ce), sb = span_of(b.cb, b.ce);
     if (sa == 0 || sb == 0)
         return false;
     if (sa == sb) {
         if (a.plane == b.plane || a.cb != b.cb || a.ce != b.ce || absdiff(a.filter, b.filter) > t.filter_tol)
             return false;
-        const double step   = dm_step(a.flo, a.fhi, tsamp);
+        const double step   = step_a;
         const double widest = static_cast<double>(max_u(a.width, b.width));
         return posfin_d(step) && dm_within_smear(a, b, t, widest, step) &&
                static_cast<double>(absdiff(a.samp, b.samp)) <= static_cast<double>(t.time_tol) * widest;
@@ -161,12 +163,12 @@ PP_HD bool on_same_curve(const Pt& a, const Pt& b, const frost_cluster_tolerance
     const Pt& narrow = sa > sb ? b : a;
     if (absdiff(wide.filter, narrow.filter) > t.filter_tol)
         return false;
-    const double step = dm_step(narrow.flo, narrow.fhi, tsamp);
+    const double step = sa > sb ? step_b : step_a;
     if (!posfin_d(step))
         return false;
     if (!dm_within_smear(wide, narrow, t, static_cast<double>(max_u(wide.width, narrow.width)), step))
         return false;
-    const double wide_step = dm_step(wide.flo, wide.fhi, tsamp);
+    const double wide_step = sa > sb ? step_a : step_b;
     if (posfin_d(wide_step) && step > 4.0 * wide_step) {
         const double expected = static_cast<double>(wide.snr) *
                                 sqrt(static_cast<double>(sa < sb ? sa : sb) / static_cast<double>(max_u(sa, sb)));
@@ -178,6 +180,10 @@ PP_HD bool on_same_curve(const Pt& a, const Pt& b, const frost_cluster_tolerance
     const double delta   = abs_d(aligned - static_cast<double>(wide.samp));
     const double widest  = static_cast<double>(max_u(wide.width, narrow.width));
     return delta <= static_cast<double>(t.time_tol) * widest;
+}
+
+PP_HD bool on_same_curve(const Pt& a, const Pt& b, const frost_cluster_tolerances& t, float tsamp) {
+    return on_same_curve(a, b, dm_step(a.flo, a.fhi, tsamp), dm_step(b.flo, b.fhi, tsamp), t, tsamp);
 }
 
 } // namespace fb::pp

@@ -35,3 +35,19 @@ def test_rows_come_back_in_order(n):
     assert np.array_equal(np.sort(got["samp_idx"]), want)
     by_sample = {int(r["peak_sample"]): float(r["snr"]) for r in rows}
     assert all(by_sample[int(g["samp_idx"])] == float(g["snr"]) for g in got)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("mode", ["TRANSITIVE", "SEEDED"])
+@pytest.mark.parametrize("n", [2, 17, 128, 129, 700, 4097])
+def test_pair_tiles_match_the_oracle(n, mode):
+    """Sub-band dedup at the edges of the pair tiles (chunks of 16 and of 128
+    rows) equals the oracle's plan, row for row."""
+    from frost_b200.postprocess import ClusterTolerances, SubbandDedupMode, SubbandDedupPlan
+    from oracle import postprocess as op
+    from tests.postprocess_cases import random_giants, same_giants
+    g = random_giants(n, n, spread=20 * n)
+    tol = ClusterTolerances(3, 3, 200, 8.0, 1e-3, 6.0)
+    m = SubbandDedupMode[mode]
+    want = op.backend("oracle").subband_dedup(g, tol, 1e-3, m)
+    assert same_giants(SubbandDedupPlan(m).execute(g, tol, 1e-3), want)
