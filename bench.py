@@ -512,7 +512,11 @@ def run_gpu(args):
         "device_bytes_served": int(st.device_bytes),
     }
     if rank == 0 and world == 1 and not args.no_cpu_baseline:
-        line["cpu_baseline"] = cpu_baseline()
+        from oracle.ref import ReferenceUnavailable
+        try:
+            line["cpu_baseline"] = cpu_baseline()
+        except ReferenceUnavailable as e:
+            line["cpu_baseline"] = {"unavailable": str(e)}
     if rank == 0:
         print(json.dumps(line), flush=True)
     if world > 1:
@@ -581,9 +585,14 @@ def run_reference(args):
     rank, world, _ = dist_env()
     if rank != 0:
         return
-    if args.warmup > 0:
-        cpu_baseline(steps=1)
-    cb = cpu_baseline(steps=args.steps)
+    from oracle.ref import ReferenceUnavailable
+    try:
+        if args.warmup > 0:
+            cpu_baseline(steps=1)
+        cb = cpu_baseline(steps=args.steps)
+    except ReferenceUnavailable as e:
+        print(json.dumps({"impl": "reference", "unavailable": str(e)}), flush=True)
+        return
     value = cb["value"]
     total = args.steps * CPU_SAMPLE * TSAMP / value
     line = {"impl": "reference", "metric": METRIC, "value": round(value, 4), "unit": UNIT,
