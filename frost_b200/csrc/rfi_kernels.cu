@@ -1342,14 +1342,98 @@ __device__ __forceinline__ float level_of(const ApplyParams& p, float loc, float
 // every measured cell from the same row, constants and clip; masks only
 // grow after it, so a cell it did not clip is never clipped here) and no
 // Kadane-along-time segment covering it. k_apply_clean writes those rows'
-// clean values (a CTA per row, no cell states, few registers) and lists
+// clean values (no cell states, few registers) and lists
 // the others; k_apply_unflagged classifies the listed rows' cells, writes
 // their values and, where a cell needs one, the fills: a row's samples and
 // cell states are staged in shared memory so neighbour draws read them
 // without touching HBM again. Masked cells are not written: the normalized
 // output zeroes them, so their fill values are never observed.
-template <int D, int V>
-__global__ void __launch_bounds__(256)
+//
+// k_apply_clean is bound by the latency of a row's loads (flags, constants,
+// samples) over the loads in flight. A CTA takes a strip of whole rows, at
+// least one and up to kStripCells groups of V channels; a thread asks for the
+// samples of its kStrip groups, one load each, before the rows' flags are
+// read. Without a transform the constants are not read at all: the cleaned
+// value is the sample. With one, more groups a thread cost registers and so
+// warps: measured over 1, 2 and 4 groups at 4 to 8 CTAs an SM, one group at 8
+// is best for a per-row term (4096 uint8 channels x 262 144 rows: 1646 us;
+// 2103 with four), two at 6 for a per-cell one (1024 float32 channels x
+// 65 536 rows: 153 us; 165 with one, 176 with four). Against a CTA a row that
+// always read the constants and single samples of the types other than uint8:
+// 1652 -> 1646 and 199 -> 153 us; without a transform 1024 uint8 channels x
+// 65 536 rows 129 -> 75 us, 1536 2-bit channels x 40 001 rows 119 -> 80 us.
+
+enum class CleanKind { kCopy, kLevel, kZdot }; // no transform; a per-row term; a per-cell one
+
+// groups of V channels that a thread holds at a time, and CTAs an SM
+template <CleanKind K> constexpr int kStrip    = K == CleanKind::kCopy ? 4 : K == CleanKind::kZdot ? 2 : 1;
+template <CleanKind K> constexpr int kStripOcc = K == CleanKind::kCopy ? 5 : K == CleanKind::kZdot ? 6 : 8;
+constexpr uint64_t kStripCells = 1024; // groups of V channels a CTA takes: whole rows, at least one
+constexpr uint64_t kStripRows = 64;
+
+__host__ __device__ inline uint64_t strip_rows(uint64_t nchans, int v) {
+    const uint64_t r = kStripCells * static_cast<uint64_t>(v) / nchans;
+    return r < 1 ? 1 : r < kStripRows ? r : kStripRows;
+}
+
+// V consecutive samples of a row as loaded: one load of 4 (from a multiple of
+// 4 channels in a row of whole groups at a 16-byte aligned block) or one
+// sample.
+template <int D, int V> struct Cells {
+    uint4 w;
+    __device__ __forceinline__ void load(const uint8_t* __restrict__ in, uint32_t c) {
+        if constexpr (V == 1) {
+            w.x = __float_as_uint(rd<D>(in, c));
+        } else if constexpr (kBitsOf<D> == 32) {
+            w = *reinterpret_cast<const uint4*>(in + 4ULL * c);
+        } else if constexpr (kBitsOf<D> == 16) {
+            const uint2 a = *reinterpret_cast<const uint2*>(in + 2ULL * c);
+            w.x = a.x;
+            w.y = a.y;
+        } else if constexpr (kBitsOf<D> == 8) {
+            w.x = *reinterpret_cast<const uint32_t*>(in + c);
+        } else if constexpr (kBitsOf<D> == 4) {
+            w.x = *reinterpret_cast<const uint16_t*>(in + c / 2);
+        } else if constexpr (kBitsOf<D> == 2) {
+            w.x = in[c / 4];
+        } else {
+            w.x = static_cast<uint32_t>(in[c / 8]) >> (c % 8);
+        }
+    }
+    __device__ __forceinline__ float at(int e) const {
+        if constexpr (V == 1)
+            return __uint_as_float(w.x);
+        else if constexpr (D == FROST_FLOAT32)
+            return __uint_as_float(e == 0 ? w.x : e == 1 ? w.y : e == 2 ? w.z : w.w);
+        else if constexpr (kBitsOf<D> == 32)
+            return static_cast<float>(e == 0 ? w.x : e == 1 ? w.y : e == 2 ? w.z : w.w);
+        else if constexpr (kBitsOf<D> == 16)
+            return static_cast<float>(((e < 2 ? w.x : w.y) >> (16 * (e & 1))) & 0xFFFFU);
+        else
+            return static_cast<float>((w.x >> (static_cast<int>(kBitsOf<D>) * e)) & ((1U << kBitsOf<D>) - 1U));
+    }
+};
+
+template <int V> __device__ __forceinline__ void load_cells(const float* __restrict__ p, float (&v)[V]) {
+    if constexpr (V == 4) {
+        const float4 a = *reinterpret_cast<const float4*>(p);
+        v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w;
+    } else {
+        v[0] = p[0];
+    }
+}
+
+template <int V> __device__ __forceinline__ void load_cells(const uint8_t* __restrict__ p, uint8_t (&v)[V]) {
+    if constexpr (V == 4) {
+        const uchar4 a = *reinterpret_cast<const uchar4*>(p);
+        v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w;
+    } else {
+        v[0] = p[0];
+    }
+}
+
+template <int D, int V, CleanKind K>
+__global__ void __launch_bounds__(256, kStripOcc<K>)
     k_apply_clean(Dims d, ApplyParams p, const uint8_t* __restrict__ raw, const float* __restrict__ loc,
                   const float* __restrict__ scale, const float* __restrict__ inv,
                   const uint8_t* __restrict__ mask, const uint8_t* __restrict__ time_flags,
@@ -1358,75 +1442,84 @@ __global__ void __launch_bounds__(256)
                   const float* __restrict__ zdot_b, const uint8_t* __restrict__ row_clip,
                   const uint8_t* __restrict__ row_kchan, float* __restrict__ work,
                   uint32_t* __restrict__ slow_rows, unsigned int* __restrict__ nslow) {
-    const uint64_t t = blockIdx.x;
-    if (t >= d.nsamps || time_flags[t] != 0)
-        return;
-    const bool row_kspec = p.kspec && (kspec_pos[t].lo >= 0 || kspec_neg[t].lo >= 0);
-    if (row_kspec || (p.narrow_active && row_clip[t] != 0) || (p.kchan && row_kchan[t] != 0)) {
-        if (threadIdx.x == 0)
-            slow_rows[atomicAdd(nslow, 1U)] = static_cast<uint32_t>(t);
-        return;
-    }
-    const uint64_t n   = d.nchans;
-    const uint32_t n32 = static_cast<uint32_t>(n);
-    const uint64_t w   = window_of(t, d.window, d.nwin);
-    const float* lw    = loc + w * n;
-    const float* sw    = scale + w * n;
-    const float* iw    = inv + w * n;
-    const uint8_t* in  = raw + t * d.row_bytes;
-    float* out         = work + t * n;
-    const float sk     = s_keep_f[t];
-    for (uint32_t cb = threadIdx.x * V; cb < n32; cb += blockDim.x * V) {
-        float xs[V], ls[V], ss[V], is[V], outv[V];
-        uint8_t ms[V];
-        if constexpr (V == 4) {
-            const float4 l4 = *reinterpret_cast<const float4*>(lw + cb);
-            const float4 s4 = *reinterpret_cast<const float4*>(sw + cb);
-            const float4 i4 = *reinterpret_cast<const float4*>(iw + cb);
-            const uchar4 m4 = *reinterpret_cast<const uchar4*>(mask + cb);
-            ls[0] = l4.x; ls[1] = l4.y; ls[2] = l4.z; ls[3] = l4.w;
-            ss[0] = s4.x; ss[1] = s4.y; ss[2] = s4.z; ss[3] = s4.w;
-            is[0] = i4.x; is[1] = i4.y; is[2] = i4.z; is[3] = i4.w;
-            ms[0] = m4.x; ms[1] = m4.y; ms[2] = m4.z; ms[3] = m4.w;
-            if constexpr (D == FROST_UINT8) {
-                const uchar4 x4 = *reinterpret_cast<const uchar4*>(in + cb);
-                xs[0] = static_cast<float>(x4.x); xs[1] = static_cast<float>(x4.y);
-                xs[2] = static_cast<float>(x4.z); xs[3] = static_cast<float>(x4.w);
-            } else {
+    constexpr int S = kStrip<K>;
+    __shared__ float sh_term[kStripRows];
+    __shared__ int sh_window[kStripRows]; // the row's window, or -1: not written here
+    const uint64_t n    = d.nchans;
+    const uint32_t n32  = static_cast<uint32_t>(n);
+    const uint64_t t0   = blockIdx.x * strip_rows(n, V);
+    const uint64_t left = d.nsamps - t0;
+    const uint32_t rows = static_cast<uint32_t>(left < strip_rows(n, V) ? left : strip_rows(n, V));
+    const uint32_t per  = n32 / V; // groups a row
+    const uint32_t all  = rows * per;
+    for (uint32_t base = 0; base < all; base += 256 * S) {
+        Cells<D, V> x[S];
+        uint32_t row[S], c[S];
 #pragma unroll
-                for (int e = 0; e < V; ++e)
-                    xs[e] = rd<D>(in, cb + e);
+        for (int k = 0; k < S; ++k) {
+            const uint32_t i = base + static_cast<uint32_t>(k) * 256 + threadIdx.x;
+            row[k]           = rows == 1 ? 0 : i / per;
+            c[k]             = (i - row[k] * per) * V;
+            if (i < all)
+                x[k].load(raw + (t0 + row[k]) * d.row_bytes, c[k]);
+        }
+        if (base == 0) {
+            if (threadIdx.x < rows) {
+                const uint64_t t     = t0 + threadIdx.x;
+                const bool row_kspec = p.kspec && (kspec_pos[t].lo >= 0 || kspec_neg[t].lo >= 0);
+                const bool slow = row_kspec || (p.narrow_active && row_clip[t] != 0) || (p.kchan && row_kchan[t] != 0);
+                int w = -1;
+                if (time_flags[t] == 0) {
+                    if (slow)
+                        slow_rows[atomicAdd(nslow, 1U)] = static_cast<uint32_t>(t);
+                    else
+                        w = static_cast<int>(window_of(t, d.window, d.nwin));
+                }
+                sh_window[threadIdx.x] = w;
+                // z less 0 is z
+                sh_term[threadIdx.x] = K == CleanKind::kCopy || p.zero_dm == FROST_ZERO_DM_OFF ? 0.0F : s_keep_f[t];
             }
-        } else {
-            ls[0] = lw[cb];
-            ss[0] = sw[cb];
-            is[0] = iw[cb];
-            ms[0] = mask[cb];
-            xs[0] = rd<D>(in, cb);
+            __syncthreads();
         }
 #pragma unroll
-        for (int e = 0; e < V; ++e) {
-            const uint32_t c = cb + e;
-            const float x    = xs[e];
-            if (ms[e] == 0) {
-                outv[e] = 0.0F;
-            } else if (is[e] == 0.0F) {
-                outv[e] = x;
-            } else {
-                const float z = (x - ls[e]) * is[e];
-                float term    = 0.0F;
-                if (p.zero_dm == FROST_ZERO_DM_SUBTRACT)
-                    term = sk;
-                else if (p.zero_dm == FROST_ZERO_DM_ZDOT)
-                    term = (zdot_a[c] * sk) + zdot_b[c];
-                const float v = z - term;
-                outv[e]       = p.transform ? level_of(p, ls[e], ss[e], v) : x;
+        for (int k = 0; k < S; ++k) {
+            const uint32_t i = base + static_cast<uint32_t>(k) * 256 + threadIdx.x;
+            const int w      = i < all ? sh_window[row[k]] : -1;
+            if (w < 0)
+                continue;
+            float ls[V], ss[V] = {}, is[V], za[V], zb[V], outv[V];
+            uint8_t ms[V];
+            const uint64_t o = static_cast<uint64_t>(w) * n + c[k];
+            load_cells<V>(mask + c[k], ms);
+            if constexpr (K != CleanKind::kCopy) {
+                load_cells<V>(loc + o, ls);
+                load_cells<V>(inv + o, is);
+                if (!p.equalize)
+                    load_cells<V>(scale + o, ss);
             }
+            if constexpr (K == CleanKind::kZdot) {
+                load_cells<V>(zdot_a + c[k], za);
+                load_cells<V>(zdot_b + c[k], zb);
+            }
+            const float sk = sh_term[row[k]];
+#pragma unroll
+            for (int e = 0; e < V; ++e) {
+                const float xe = x[k].at(e);
+                float v        = xe;
+                if constexpr (K != CleanKind::kCopy) {
+                    const float z    = (xe - ls[e]) * is[e];
+                    const float term = K == CleanKind::kZdot ? (za[e] * sk) + zb[e] : sk;
+                    if (is[e] != 0.0F)
+                        v = level_of(p, ls[e], ss[e], z - term);
+                }
+                outv[e] = ms[e] == 0 ? 0.0F : v;
+            }
+            float* out = work + (t0 + row[k]) * n + c[k];
+            if constexpr (V == 4)
+                *reinterpret_cast<float4*>(out) = make_float4(outv[0], outv[1], outv[2], outv[3]);
+            else
+                out[0] = outv[0];
         }
-        if constexpr (V == 4)
-            *reinterpret_cast<float4*>(out + cb) = make_float4(outv[0], outv[1], outv[2], outv[3]);
-        else
-            out[cb] = outv[0];
     }
 }
 
@@ -2242,27 +2335,36 @@ void launch_apply_unflagged(const Dims& d, const ApplyParams& p, const uint8_t* 
         return;
     if (d.nchans >= (uint64_t{1} << 31) || d.nsamps >= (uint64_t{1} << 31))
         throw Error(FROST_ERR_INVALID_ARGUMENT, "apply: too many channels or samples for one block");
-    // 4-channel vectors need nchans % 4 == 0 and, for the byte loads of the
-    // raw row, a 4-byte aligned block
-    const bool vec = d.nchans % 4 == 0 && reinterpret_cast<uintptr_t>(raw) % 4 == 0;
+    // 4-channel vectors need nchans % 4 == 0 and, for the loads of 4 samples of
+    // the raw row, an aligned block (the cleaner's always is)
+    const bool vec = d.nchans % 4 == 0 && aligned16(raw);
+    const CleanKind kind = !p.transform                         ? CleanKind::kCopy
+                           : p.zero_dm == FROST_ZERO_DM_ZDOT ? CleanKind::kZdot
+                                                              : CleanKind::kLevel;
     int dev = 0, sms = 0;
     FB_CUDA(cudaGetDevice(&dev));
     FB_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
     // the listed rows: a few CTAs an SM loop over them (the count is read on the device)
     const unsigned slow_grid = static_cast<unsigned>(std::min<uint64_t>(d.nsamps, static_cast<uint64_t>(sms) * 4));
     FB_DISPATCH(d.dtype, {
-        if (vec) {
-            k_apply_clean<D, 4><<<static_cast<unsigned>(d.nsamps), 256, 0, s>>>(
+        auto clean = [&](auto vtag) {
+            constexpr int V = decltype(vtag)::value;
+            const auto k    = kind == CleanKind::kCopy    ? &k_apply_clean<D, V, CleanKind::kCopy>
+                              : kind == CleanKind::kLevel ? &k_apply_clean<D, V, CleanKind::kLevel>
+                                                          : &k_apply_clean<D, V, CleanKind::kZdot>;
+            const uint64_t rows = strip_rows(d.nchans, V);
+            k<<<static_cast<unsigned>((d.nsamps + rows - 1) / rows), 256, 0, s>>>(
                 d, p, raw, loc, scale, inv, mask, time_flags, kspec_pos, kspec_neg, s_keep_f, zdot_a, zdot_b,
                 row_clip, row_kchan, work, slow_rows, nslow);
+        };
+        if (vec) {
+            clean(std::integral_constant<int, 4>{});
             set_smem(reinterpret_cast<const void*>(&k_apply_unflagged<D, 4>), smem);
             k_apply_unflagged<D, 4><<<slow_grid, 256, smem, s>>>(
                 d, p, raw, loc, scale, inv, mask, time_flags, kspec_pos, kspec_neg, kchan_pos,
                 kchan_neg, kchan_any, s_keep_f, zdot_a, zdot_b, slow_rows, nslow, work, counters);
         } else {
-            k_apply_clean<D, 1><<<static_cast<unsigned>(d.nsamps), 256, 0, s>>>(
-                d, p, raw, loc, scale, inv, mask, time_flags, kspec_pos, kspec_neg, s_keep_f, zdot_a, zdot_b,
-                row_clip, row_kchan, work, slow_rows, nslow);
+            clean(std::integral_constant<int, 1>{});
             set_smem(reinterpret_cast<const void*>(&k_apply_unflagged<D, 1>), smem);
             k_apply_unflagged<D, 1><<<slow_grid, 256, smem, s>>>(
                 d, p, raw, loc, scale, inv, mask, time_flags, kspec_pos, kspec_neg, kchan_pos,

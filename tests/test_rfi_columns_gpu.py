@@ -236,3 +236,23 @@ def test_scans_do_not_depend_on_the_sample_type(nchans, nsamps, zdot):
         out.append((rep[0],) + tuple(rep[1][k] for k in ("samps_kadane", "cells_kadane_spectrum",
                                                          "cells_kadane_channel", "samps_broad", "chans_dead")))
     assert out[0] == out[1] == out[2]
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("nchans,nsamps", [(8, 200), (56, 131), (1000, 70), (1029, 67), (4104, 66)])
+@pytest.mark.parametrize("dtype,bits", [(DataType.UINT1, 1), (DataType.UINT2, 2), (DataType.UINT4, 4), (DataType.UINT8, 8),
+                                        (DataType.UINT16, 16), (DataType.UINT32, 24), (DataType.FLOAT32, 0)])
+def test_clean_rows_are_written_as_read(nchans, nsamps, dtype, bits):
+    """Strips of many rows, of one and of a part of one, whole and partial;
+    groups of four samples of each width and single ones."""
+    from frost_b200.rfi import RFICleaner
+    if nchans * max(bits, 1) % 8 != 0 and bits < 8 and bits != 0:
+        pytest.skip("rows are whole bytes")
+    rng = np.random.default_rng(nchans + nsamps + bits)
+    x = (rng.normal(0, 3, (nsamps, nchans)) if bits == 0 else rng.integers(0, 2 ** bits, (nsamps, nchans))).astype(np.float32)
+    gpu = RFICleaner(RfiConfig.quiet(), BlockLayout(nchans, nsamps, dtype, 2.0 ** -10, 1400.0, 1.0), 32.0)
+    got = gpu.execute_normalized(pack(x, dtype))
+    level, scale = bandpass(x)
+    with np.errstate(divide="ignore", invalid="ignore"):
+        want = np.ascontiguousarray(((x - level) * (np.float32(1) / scale)).T)
+    assert same_measured(got, want, [((0, nsamps), scale)])
