@@ -1359,9 +1359,10 @@ __device__ __forceinline__ float level_of(const ApplyParams& p, float loc, float
 // is best for a per-row term (4096 uint8 channels x 262 144 rows: 1646 us;
 // 2103 with four), two at 6 for a per-cell one (1024 float32 channels x
 // 65 536 rows: 153 us; 165 with one, 176 with four). Against a CTA a row that
-// always read the constants and single samples of the types other than uint8:
-// 1652 -> 1646 and 199 -> 153 us; without a transform 1024 uint8 channels x
-// 65 536 rows 129 -> 75 us, 1536 2-bit channels x 40 001 rows 119 -> 80 us.
+// always read the constants, and samples one by one for types other than
+// uint8: 1620 -> 1646 and 228 -> 153 us; without a transform 1024 uint8
+// channels x 65 536 rows 132 -> 75 us, 1536 2-bit channels x 40 001 rows
+// 90 -> 80 us.
 
 enum class CleanKind { kCopy, kLevel, kZdot }; // no transform; a per-row term; a per-cell one
 
