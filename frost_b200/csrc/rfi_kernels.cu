@@ -748,27 +748,6 @@ constexpr int kScanRows = 128; // rows per CTA (one thread each)
 
 template <int D> constexpr bool kIntRow = D != FROST_FLOAT32 && kBitsOf<D> <= 16;
 
-/** KadaneBest::append for the values of a row: the same best run from fewer
- * operations. The values are floats, so a sum that is not zero is at least
- * 2^-149: its high word tells its sign and whether it is zero. A run's start
- * is taken at every position before which the open run is empty (the run it
- * starts, if any, starts there). Appending 0 for a channel that is skipped
- * changes no run: an open run keeps its sum and the comparisons are strict. */
-struct RowRuns {
-    double ssum = 0.0, bsum = 0.0;
-    int32_t sstart = 0, bstart = 0, bend = -1;
-    __device__ __forceinline__ void append(int32_t i, double u) {
-        const double s = ssum + u;
-        sstart         = __double2hiint(ssum) == 0 ? i : sstart;
-        ssum           = __double2hiint(s) > 0 ? s : 0.0;
-        const bool up  = ssum > bsum;
-        bsum           = up ? ssum : bsum;
-        bstart         = up ? sstart : bstart;
-        bend           = up ? i : bend;
-    }
-    __device__ Run best() const { return {bsum, bstart, bend}; }
-};
-
 // One row of the row scan (lib/cpu/rfi_cpu_measure.cpp:305-446), fed its
 // channels in ascending order: the detection series sums and the Kadane
 // states across frequency.
@@ -782,7 +761,7 @@ struct ScanRowAcc {
     uint64_t isx = 0, isxx = 0;
     uint32_t tsx = 0, tsxx = 0;      // W32: the current tile's integer sums
     uint32_t n_keep = 0, n_meas = 0; // counts (exact as doubles when used)
-    RowRuns sp, sn; // rows are scanned whole: only the best runs are needed
+    KadaneBest sp, sn; // rows are scanned whole: only the best runs are needed
     // Channel c, x its sample and xi the integer code (INT: x == xi exactly).
     // A channel that is not used adds 0 everywhere: no branch stands between
     // one channel's sums and the next one's, and a sum that starts at +0 is
@@ -881,7 +860,7 @@ struct ScanRowAcc {
 // 1912 uint8 channels (pitch no multiple of 16) x 4289 rows 540 -> 99 us,
 // 1536 2-bit x 40 001: 236 -> 122, against a branch a channel and rows
 // decoded one sample at a time; 4096 x 262 144 with Kadane across frequency
-// 2550 -> 2520 (selects on the integer pipe bound it).
+// 2550 -> 2460 (selects on the integer pipe bound it).
 template <int U> constexpr int kRowStride = U == 16 ? 144 : 132;
 constexpr int kRowTileBytes = 128;
 template <int D> constexpr int kRowTiles = kBitsOf<D> == 32 ? 3 : 2;
@@ -1016,74 +995,13 @@ __global__ void __launch_bounds__(kScanRows)
                    kspec_whole, row_clip);
 }
 
-/** KadanePair32 (the states of u and -u appended together) in fewer
- * operations, for values that are floats: a sum's high word tells its sign
- * and whether it is zero (RowRuns), and an open run's start is taken at
- * every position before which it is empty (an empty run's is set when the
- * state is stored). */
-struct ColRuns {
-    struct Side {
-        double psum = 0.0, ssum = 0.0, bsum = 0.0;
-        int32_t pend = -1, sstart = 0, bstart = 0, bend = -1;
-        __device__ __forceinline__ void begin(int32_t i) {
-            pend   = i - 1;
-            bstart = i;
-            bend   = i - 1;
-        }
-        __device__ __forceinline__ void append(int32_t i, double total, double u) {
-            const bool longer = total > psum; // the prefix runs start at `first`
-            psum              = longer ? total : psum;
-            pend              = longer ? i : pend;
-            const double s    = ssum + u;
-            sstart            = __double2hiint(ssum) == 0 ? i : sstart;
-            ssum              = __double2hiint(s) > 0 ? s : 0.0;
-            const bool up     = ssum > bsum;
-            bsum              = up ? ssum : bsum;
-            bstart            = up ? sstart : bstart;
-            bend              = up ? i : bend;
-        }
-    };
-    double total = 0.0; // of u
-    int32_t first = 0;
-    bool empty    = true;
-    Side pos, neg;
-
-    __device__ __forceinline__ void begin(int32_t i) {
-        empty = false;
-        first = i;
-        pos.begin(i);
-        neg.begin(i);
-    }
-    __device__ __forceinline__ void append(int32_t i, double u) {
-        total += u;
-        pos.append(i, total, u);
-        neg.append(i, -total, -u);
-    }
-    /** The state of u (NEG: of -u, its total 0 - total) after appends up to
-     * position `last`. */
-    template <bool NEG> __device__ KadaneState widen(int32_t last) const {
-        KadaneState k = KadaneState::make();
-        if (empty)
-            return k;
-        const Side& sd = NEG ? neg : pos;
-        k.total  = NEG ? 0.0 - total : total;
-        k.first  = first;
-        k.last   = last;
-        k.empty  = 0;
-        k.prefix = {sd.psum, first, sd.pend};
-        k.suffix = {sd.ssum, sd.ssum == 0.0 ? last + 1 : sd.sstart, last};
-        k.best   = {sd.bsum, sd.bstart, sd.bend};
-        return k;
-    }
-};
-
 // One (chunk, channel) sequence of the column scan
 // (lib/cpu/rfi_cpu_measure.cpp:305-446): the block min/max of unmeasured
 // cells, zdot sums and Kadane-along-time states. The per-(window, channel)
 // constants are reloaded only when the window changes; rows are taken a few
 // at a time, without a branch where they lie in one window and the channel is
 // measured there.
-// With Kadane: 4096 uint8 channels x 262 144 rows 3150 -> 2225 us, 479 float32
+// With Kadane: 4096 uint8 channels x 262 144 rows 3150 -> 2095 us, 479 float32
 // channels x 12 734 rows 193 -> 70.
 template <bool ZDOT, bool KCHAN>
 struct ScanColAcc {
@@ -1100,7 +1018,7 @@ struct ScanColAcc {
     float cmin = FLT_MAX, cmax = -FLT_MAX;
     ZdotSums zs{0, 0, 0, 0, 0};
     uint32_t zn = 0;
-    ColRuns kk; // Kadane along time of u and -u, widened when stored
+    KadanePair32 kk; // Kadane along time of u and -u, widened when stored
     // the first sample of an active channel's chunk (every later sample of
     // the chunk follows in order)
     __device__ __forceinline__ void begin(uint64_t t0) {
@@ -1171,8 +1089,8 @@ struct ScanColAcc {
             // an active channel appended every sample of the chunk
             const uint64_t t1   = (k + 1) * d->chunk < d->nsamps ? (k + 1) * d->chunk : d->nsamps;
             const int32_t last  = static_cast<int32_t>(t1) - 1;
-            kp_out[o] = kk.template widen<false>(last);
-            kn_out[o] = kk.template widen<true>(last);
+            kp_out[o] = kk.widen_pos(last);
+            kn_out[o] = kk.widen_neg(last);
         }
     }
 };

@@ -11,6 +11,7 @@
 #pragma once
 
 #include <cstdint>
+#include <cstring>
 
 #if defined(__CUDACC__)
 #define FB_HD __host__ __device__ __forceinline__
@@ -220,61 +221,91 @@ struct KadaneState32 {
     }
 };
 
-/** The two KadaneState32 of one sequence u and its negation -u, appended
- * together from a known first position (`begin`) with 32-bit positions:
- * the states of -u share the running total (negated: the sums of -u are
- * the exact negations of those of u) and compare it for their own best
- * prefix; the open runs' ends are the last position (`widen_*(last)`). The
- * same sums, comparisons and runs as two KadaneState32 appends. */
+/** Whether a sum of floats is greater than zero, from its high word: 1 ..
+ * 0x7FF00000 there means positive or +inf. Such a sum is a multiple of
+ * 2^-149, so one with a zero high word is zero; a negative one has the sign
+ * bit set; a NaN (0 x inf of a channel whose scale has no float inverse) is
+ * above +inf and, as in a comparison, not greater than zero. */
+FB_HD bool positive_sum(double s) {
+#if defined(__CUDA_ARCH__)
+    const uint32_t hi = static_cast<uint32_t>(__double2hiint(s));
+#else
+    uint64_t bits;
+    std::memcpy(&bits, &s, sizeof(bits));
+    const uint32_t hi = static_cast<uint32_t>(bits >> 32U);
+#endif
+    return hi - 1U < 0x7FF00000U;
+}
+
+/** The open (suffix) and the best run of a sequence of floats: KadaneState's
+ * sums, comparisons and runs from fewer operations, without branches. The
+ * open run ends at the position just appended; its start is taken at every
+ * position before which it is empty (the run it starts, if any, starts
+ * there). Appending 0 changes no run. */
+struct OpenBestRun {
+    double ssum = 0.0, bsum = 0.0;
+    int32_t sstart = 0, bstart = 0, bend = -1;
+    bool open = false; // ssum > 0
+
+    FB_HD void append(int32_t i, double u) {
+        const double s = ssum + u;
+        sstart         = open ? sstart : i;
+        open           = positive_sum(s);
+        ssum           = open ? s : 0.0;
+        const bool up  = ssum > bsum;
+        bsum           = up ? ssum : bsum;
+        bstart         = up ? sstart : bstart;
+        bend           = up ? i : bend;
+    }
+};
+
+/** The best run of KadaneState::append over a sequence of floats that is
+ * never combined with another. When no run ever has a positive sum the best
+ * run is empty (length 0) and reported at position 0 rather than at the
+ * first position appended; callers use only a best run's length when it is
+ * empty. */
+struct KadaneBest : OpenBestRun {
+    FB_HD Run best() const { return {bsum, bstart, bend}; }
+};
+
+/** The KadaneStates of a sequence u of floats and of its negation -u,
+ * appended together from a known first position (`begin`): the states of -u
+ * share the running total (negated: the sums of -u are the exact negations
+ * of those of u) and compare it for their own best prefix; the prefix runs
+ * start at the first position. */
 struct KadanePair32 {
     struct Side {
-        double psum = 0.0, ssum = 0.0, bsum = 0.0;
-        int32_t pend = -1, sstart = 0, bstart = 0, bend = -1;
+        double psum = 0.0;
+        int32_t pend = -1;
+        OpenBestRun run;
+
+        FB_HD void begin(int32_t i) {
+            pend       = i - 1;
+            run.bstart = i;
+            run.bend   = i - 1;
+        }
+        FB_HD void append(int32_t i, double total, double u) {
+            const bool longer = total > psum;
+            psum              = longer ? total : psum;
+            pend              = longer ? i : pend;
+            run.append(i, u);
+        }
     };
     double total = 0.0; // of u
     int32_t first = 0;
     bool empty    = true;
     Side pos, neg;
 
-    FB_HD static void begin_side(Side& sd, int32_t i) {
-        sd.pend   = i - 1;
-        sd.sstart = i;
-        sd.bstart = i;
-        sd.bend   = i - 1;
-    }
     FB_HD void begin(int32_t i) {
         empty = false;
         first = i;
-        begin_side(pos, i);
-        begin_side(neg, i);
-    }
-    FB_HD static void open_run(Side& sd, int32_t i, double s) {
-        if (s > 0.0) {
-            if (sd.ssum == 0.0)
-                sd.sstart = i;
-            sd.ssum = s;
-        } else {
-            sd.ssum   = 0.0;
-            sd.sstart = i + 1;
-        }
-        if (sd.ssum > sd.bsum) {
-            sd.bsum   = sd.ssum;
-            sd.bstart = sd.sstart;
-            sd.bend   = i;
-        }
+        pos.begin(i);
+        neg.begin(i);
     }
     FB_HD void append(int32_t i, double u) {
         total += u;
-        if (total > pos.psum) { // the prefix runs start at `first`
-            pos.psum = total;
-            pos.pend = i;
-        }
-        if (-total > neg.psum) {
-            neg.psum = -total;
-            neg.pend = i;
-        }
-        open_run(pos, i, pos.ssum + u);
-        open_run(neg, i, neg.ssum - u);
+        pos.append(i, total, u);
+        neg.append(i, -total, -u);
     }
     FB_HD KadaneState widen(const Side& sd, double tot, int32_t last) const {
         KadaneState k = KadaneState::make();
@@ -285,8 +316,8 @@ struct KadanePair32 {
         k.last   = last;
         k.empty  = 0;
         k.prefix = {sd.psum, first, sd.pend};
-        k.suffix = {sd.ssum, sd.sstart, last};
-        k.best   = {sd.bsum, sd.bstart, sd.bend};
+        k.suffix = {sd.run.ssum, sd.run.open ? sd.run.sstart : last + 1, last};
+        k.best   = {sd.run.bsum, sd.run.bstart, sd.run.bend};
         return k;
     }
     /** The state of u after appends up to position `last`. */
@@ -294,36 +325,6 @@ struct KadanePair32 {
     /** The state of -u (its total is 0 - total: +0 rather than -0 for a
      * zero total, as the sum of -u would be). */
     FB_HD KadaneState widen_neg(int32_t last) const { return widen(neg, 0.0 - total, last); }
-};
-
-/** The best run of KadaneState::append over a sequence that is never
- * combined with another: only the open (suffix) run and the best one are
- * kept, with 32-bit positions. The open run always ends at the position
- * just appended and is empty exactly when its sum is zero. When no run
- * ever has a positive sum the best run is empty (length 0) and reported at
- * position 0 rather than at the first position appended; callers use only
- * a best run's length when it is empty. */
-struct KadaneBest {
-    double ssum = 0.0, bsum = 0.0;
-    int32_t sstart = 0, bstart = 0, bend = -1;
-
-    FB_HD void append(int32_t i, double u) {
-        const double s = ssum + u;
-        if (s > 0.0) {
-            if (ssum == 0.0)
-                sstart = i;
-            ssum = s;
-        } else {
-            ssum   = 0.0;
-            sstart = i + 1;
-        }
-        if (ssum > bsum) {
-            bsum   = ssum;
-            bstart = sstart;
-            bend   = i;
-        }
-    }
-    FB_HD Run best() const { return {bsum, bstart, bend}; }
 };
 
 /** Largest power of five not above `count` (0 for 0). */
