@@ -5,6 +5,8 @@
 // (docs/architecture.md:78-80, lib/cuda/gpu_utils.cuh:13-20).
 #pragma once
 
+#include <array>
+#include <atomic>
 #include <cstddef>
 #include <cstdint>
 #include <mutex>
@@ -70,6 +72,20 @@ inline void allow_large_smem(const void* fn) {
     FB_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  optin - static_cast<int>(a.sharedSizeBytes)));
     done.insert({fn, dev});
+}
+
+/** SMs of the calling thread's current device. */
+inline unsigned sm_count() {
+    static std::array<std::atomic<int>, 64> known{}; // by device; 0: not asked yet
+    int dev = 0;
+    FB_CUDA(cudaGetDevice(&dev));
+    int sms = static_cast<size_t>(dev) < known.size() ? known[dev].load(std::memory_order_relaxed) : 0;
+    if (sms == 0) {
+        FB_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+        if (static_cast<size_t>(dev) < known.size())
+            known[dev].store(sms, std::memory_order_relaxed);
+    }
+    return static_cast<unsigned>(sms);
 }
 #define FB_LAUNCH_CHECK() ::fb::cuda_check(cudaGetLastError(), "kernel launch", __FILE__, __LINE__)
 

@@ -968,10 +968,7 @@ __global__ void __launch_bounds__(256)
 }
 
 unsigned copy_blocks(size_t n) {
-    int dev = 0, sms = 0;
-    FB_CUDA(cudaGetDevice(&dev));
-    FB_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-    return static_cast<unsigned>(std::min<size_t>((n + 255) / 256, static_cast<size_t>(sms) * 8));
+    return static_cast<unsigned>(std::min<size_t>((n + 255) / 256, size_t{8} * sm_count()));
 }
 
 void copy_floats(float* dst, size_t dpitch, const float* src, size_t spitch, size_t width, size_t rows,

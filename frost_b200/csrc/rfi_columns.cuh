@@ -22,6 +22,7 @@
 
 #include <cstdint>
 
+#include "common.hpp"
 #include "rfi_stage.cuh"
 
 namespace fb::rfi::cols {
@@ -81,7 +82,7 @@ constexpr int kAhead = 8;  // rows its loads run ahead
 // groups an SM: the Welford walk 1719 us with one, 1350 us with four; 1024
 // channels x 2 windows: 690 us with one).
 constexpr int kManyGroups = 4;
-__host__ __device__ constexpr bool few_groups(uint64_t groups) { return groups <= 2 * 148; }
+inline bool few_groups(uint64_t groups) { return groups <= 2 * sm_count(); }
 
 /** Rows [0, n) of a 32-channel segment of BITS-bit samples, row r at
  * src + r * pitch. U: bytes a copy (16 or 4); S stages of H rows; SIDE: a

@@ -46,7 +46,7 @@ constexpr int kMaxVoteSlots     = 128;
 
 unsigned grid_for(uint64_t n, unsigned block) {
     const uint64_t g = (n + block - 1) / block;
-    return static_cast<unsigned>(std::max<uint64_t>(std::min<uint64_t>(g, 148ULL * 64), 1));
+    return static_cast<unsigned>(std::max<uint64_t>(std::min<uint64_t>(g, uint64_t{64} * sm_count()), 1));
 }
 
 uint64_t pow2_at_least(uint64_t n) {

@@ -2061,7 +2061,7 @@ void launch_check_finite(const uint8_t* raw, uint64_t nwords, unsigned long long
     if (nwords == 0)
         return;
     const uint64_t head   = std::min<uint64_t>(nwords, (16 - reinterpret_cast<uintptr_t>(raw) % 16) % 16 / 4);
-    const unsigned blocks = static_cast<unsigned>(std::min<uint64_t>((nwords + 4095) / 4096, 148 * 8));
+    const unsigned blocks = static_cast<unsigned>(std::min<uint64_t>((nwords + 4095) / 4096, 8 * sm_count()));
     k_check_finite<<<blocks, 256, 0, s>>>(reinterpret_cast<const uint32_t*>(raw), nwords, head, first_bad);
     FB_COUNT_LAUNCH();
 }
@@ -2069,7 +2069,7 @@ void launch_check_finite(const uint8_t* raw, uint64_t nwords, unsigned long long
 void launch_begin(const Dims& d, unsigned long long* counters, uint64_t nslots, uint32_t* unmeasured,
                   uint8_t* kchan_any, uint8_t* time_flags, uint8_t* row_kchan, unsigned int* nslow, cudaStream_t s) {
     const uint64_t most   = std::max({nslots, d.nchans, d.nsamps, uint64_t{1}});
-    const unsigned blocks = static_cast<unsigned>(std::min<uint64_t>((most + 255) / 256, 148 * 4));
+    const unsigned blocks = static_cast<unsigned>(std::min<uint64_t>((most + 255) / 256, 4 * sm_count()));
     k_begin<<<blocks, 256, 0, s>>>(counters, nslots, unmeasured, kchan_any, d.nchans, time_flags, row_kchan, d.nsamps,
                                    nslow);
     FB_COUNT_LAUNCH();
@@ -2260,11 +2260,8 @@ void launch_apply_unflagged(const Dims& d, const ApplyParams& p, const uint8_t* 
     const CleanKind kind = !p.transform                         ? CleanKind::kCopy
                            : p.zero_dm == FROST_ZERO_DM_ZDOT ? CleanKind::kZdot
                                                               : CleanKind::kLevel;
-    int dev = 0, sms = 0;
-    FB_CUDA(cudaGetDevice(&dev));
-    FB_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
     // the listed rows: a few CTAs an SM loop over them (the count is read on the device)
-    const unsigned slow_grid = static_cast<unsigned>(std::min<uint64_t>(d.nsamps, static_cast<uint64_t>(sms) * 4));
+    const unsigned slow_grid = static_cast<unsigned>(std::min<uint64_t>(d.nsamps, 4 * sm_count()));
     FB_DISPATCH(d.dtype, {
         auto clean = [&](auto vtag) {
             constexpr int V = decltype(vtag)::value;
@@ -2301,7 +2298,7 @@ void launch_apply_flagged(const Dims& d, const ApplyParams& p, const uint64_t* f
     if (d.nsamps == 0)
         return;
     const size_t smem     = d.nchans * (sizeof(float) + 1);
-    const unsigned blocks = static_cast<unsigned>(std::min<uint64_t>(d.nsamps, 148 * 8));
+    const unsigned blocks = static_cast<unsigned>(std::min<uint64_t>(d.nsamps, 8 * sm_count()));
     set_smem(reinterpret_cast<const void*>(&k_apply_flagged), smem);
     k_apply_flagged<<<blocks, 256, smem, s>>>(d, p, flagged, nflagged, loc, scale, inv, mask, time_flags, work,
                                               counters);
@@ -2312,7 +2309,7 @@ void launch_unpack(const Dims& d, const uint8_t* raw, float* work, cudaStream_t 
     const uint64_t total = d.nsamps * d.nchans;
     if (total == 0)
         return;
-    const unsigned blocks = static_cast<unsigned>(std::min<uint64_t>((total + 255) / 256, 148 * 32));
+    const unsigned blocks = static_cast<unsigned>(std::min<uint64_t>((total + 255) / 256, 32 * sm_count()));
     FB_DISPATCH(d.dtype, k_unpack<D><<<blocks, 256, 0, s>>>(d, raw, work));
     FB_COUNT_LAUNCH();
 }

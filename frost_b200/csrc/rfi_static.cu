@@ -220,7 +220,7 @@ void normalize_static(const frost_block_layout& layout, float baseline_length, c
         const uint64_t words     = valid * n;
         unsigned long long first = words;
         FB_CUDA(cudaMemcpyAsync(first_bad, &first, sizeof(first), cudaMemcpyHostToDevice, stream));
-        const unsigned blocks = static_cast<unsigned>(std::min<uint64_t>((words + 255) / 256, 148 * 16));
+        const unsigned blocks = static_cast<unsigned>(std::min<uint64_t>((words + 255) / 256, 16 * sm_count()));
         k_find_nonfinite<<<blocks, 256, 0, stream>>>(reinterpret_cast<const uint32_t*>(block), words,
                                                      first_bad);
         FB_LAUNCH_CHECK();

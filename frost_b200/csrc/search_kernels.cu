@@ -1677,7 +1677,7 @@ void launch_frontier(const RunState* carry, int64_t n, unsigned long long sample
     FB_LAUNCH_CHECK();
     if (n == 0)
         return;
-    const auto blocks = static_cast<unsigned>(std::min<int64_t>((n + 255) / 256, 4 * 148));
+    const auto blocks = static_cast<unsigned>(std::min<int64_t>((n + 255) / 256, 4 * sm_count()));
     k_frontier<<<blocks, 256, 0, s>>>(carry, n, out);
     FB_LAUNCH_CHECK();
 }
@@ -1766,7 +1766,7 @@ void launch_cand_range(const frost_candidate* c, const unsigned long long* count
                        unsigned long long* range, cudaStream_t s) {
     FB_CUDA(cudaMemsetAsync(range, 0xFF, sizeof(unsigned long long), s));
     FB_CUDA(cudaMemsetAsync(range + 1, 0, sizeof(unsigned long long), s));
-    const uint64_t grid = std::min<uint64_t>(blocks256(cap), 4 * 148);
+    const uint64_t grid = std::min<uint64_t>(blocks256(cap), 4 * sm_count());
     k_cand_range<<<static_cast<unsigned>(grid), 256, 0, s>>>(c, count, cap, range);
     FB_LAUNCH_CHECK();
 }
