@@ -75,14 +75,20 @@ __device__ __forceinline__ void cp_async4(void* dst, const void* src, int n) {
 constexpr int kBatch = 16; // rows a walker takes without a branch
 constexpr int kAhead = 8;  // rows its loads run ahead
 
-// Groups a CTA holds. One while the groups are no more than two an SM: a
-// walker then has a scheduler to itself. Four from there on: the warps of a
-// CTA go to the schedulers in turn, so one walker in every two-warp CTA would
-// leave half of the schedulers to the feeders (4096 channels x 8 windows, 7
-// groups an SM: the Welford walk 1719 us with one, 1350 us with four; 1024
-// channels x 2 windows: 690 us with one).
-constexpr int kManyGroups = 4;
-inline bool few_groups(uint64_t groups) { return groups <= 2 * sm_count(); }
+// Groups a CTA holds: one while the groups are no more than so many an SM, as
+// a walker then has a scheduler to itself, and four from there on, as the
+// warps of a CTA go to the schedulers in turn, so that one walker in every
+// two-warp CTA leaves half of the schedulers to the feeders. Measured at
+// windows of 31 250 rows on both sides of each line, one group : four, us, by
+// groups an SM:
+//   bandpass  2.2: 186 : 276, 3.9: 190 : 282, 5.2: 270 : 325 | 6.9: 369 : 333,
+//             10.4: 526 : 400 (12.1: 613 : 670, four's second wave)
+//   moments   uint8: 1.9: 612 : 659 | 2.2: 870 : 659, 3.9: 960 : 672, 6.9: 1756 : 1172;
+//             float32: 1.9: 562 : 835 | 2.2: 775 : 839, 3.0: 844 : 842, 6.9: 1584 : 1317
+//   Welford   1.9: 643 : 801, 3.9: 763 : 804 | 5.2: 1017 : 965, 6.9: 1550 : 971
+constexpr int kManyGroups     = 4;
+constexpr uint64_t kBandpassFew = 6, kMomentsFew = 2, kWelfordFew = 4;
+inline bool few_groups(uint64_t groups, uint64_t per_sm) { return groups <= per_sm * sm_count(); }
 
 /** Rows [0, n) of a 32-channel segment of BITS-bit samples, row r at
  * src + r * pitch. U: bytes a copy (16 or 4); S stages of H rows; SIDE: a

@@ -259,9 +259,10 @@ __global__ void k_sample_rows(Dims d, const uint8_t* __restrict__ raw, float* __
 // per channel, and warp 0 finishes the tree over the <= 25 block values. The
 // level goes to loc and a flat flag (every sampled value of the channel
 // compares equal) to inv; a second sweep takes the scale, remedian(|x -
-// level|) x 1.4826 (lib/cpu/spectra_cpu.cpp:73-130). 25 warps, one a block,
-// where channel groups are few (load latency bounds them: 64 channels 33 +
-// 20 us with 8 warps and two launches, 16 here), else 8.
+// level|) x 1.4826 (lib/cpu/spectra_cpu.cpp:73-130). 25 warps, one a block:
+// load latency bounds them (64 channels 33 + 20 us with 8 warps and two
+// launches, 16 here; 1024 channels x 32 windows 297 us with 8 warps, 168 here).
+constexpr int kRemedianWarps = 25;
 
 // The remedian of 25 values p[0], p[stride], ... (medians of five
 // consecutive values, then their median): the 25 loads are issued together
@@ -331,7 +332,7 @@ __device__ __forceinline__ float remedian125(const float* __restrict__ p, uint64
 
 /** The 32 channels' remedian over the window's sampled rows (ABS: of |x -
  * level|) in warp 0's lanes; lo, hi the range of this warp's values. */
-template <bool ABS, int W>
+template <bool ABS>
 __device__ __forceinline__ float remedian_rows(const float* __restrict__ src, uint64_t n, int levels, bool in,
                                                float level, float (&part)[25][32], float& lo, float& hi) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -339,7 +340,7 @@ __device__ __forceinline__ float remedian_rows(const float* __restrict__ src, ui
     const int up       = levels - kb;             // levels over the blocks (0..2)
     const int nblk     = up == 0 ? 1 : up == 1 ? 5 : 25;
     const uint64_t blk = kb == 1 ? 5 : kb == 2 ? 25 : 125; // a window has 5 rows or more
-    for (int b = warp; b < nblk; b += W) {
+    for (int b = warp; b < nblk; b += kRemedianWarps) {
         const float* p = src + static_cast<uint64_t>(b) * blk * n;
         float v        = 0.0F;
         if (in) {
@@ -366,12 +367,11 @@ __device__ __forceinline__ float remedian_rows(const float* __restrict__ src, ui
     return r;
 }
 
-template <int W>
-__global__ void __launch_bounds__(32 * W)
+__global__ void __launch_bounds__(32 * kRemedianWarps)
     k_remedian(Dims d, const float* __restrict__ samples, float* __restrict__ loc, float* __restrict__ scale,
                float* __restrict__ flat_out) {
     __shared__ float part[25][32];
-    __shared__ float plo[W][32], phi[W][32];
+    __shared__ float plo[kRemedianWarps][32], phi[kRemedianWarps][32];
     __shared__ float level_of[32];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const uint64_t n = d.nchans;
@@ -386,18 +386,18 @@ __global__ void __launch_bounds__(32 * W)
     const uint64_t o = w * n + c;
     const float* src = samples + w * kMaxBandpassRows * n + (in ? c : 0);
     float lo = FLT_MAX, hi = -FLT_MAX, ignored_lo = 0.0F, ignored_hi = 0.0F;
-    const float level = remedian_rows<false, W>(src, n, levels, in, 0.0F, part, lo, hi);
+    const float level = remedian_rows<false>(src, n, levels, in, 0.0F, part, lo, hi);
     plo[warp][lane]   = lo;
     phi[warp][lane]   = hi;
     if (warp == 0)
         level_of[lane] = level;
     __syncthreads();
-    const float r = remedian_rows<true, W>(src, n, levels, in, level_of[lane], part, ignored_lo, ignored_hi);
+    const float r = remedian_rows<true>(src, n, levels, in, level_of[lane], part, ignored_lo, ignored_hi);
     if (warp != 0 || !in)
         return;
     float a = plo[0][lane], z = phi[0][lane];
 #pragma unroll
-    for (int k = 1; k < W; ++k) {
+    for (int k = 1; k < kRemedianWarps; ++k) {
         a = fminf(a, plo[k][lane]);
         z = fmaxf(z, phi[k][lane]);
     }
@@ -2041,11 +2041,12 @@ static void set_smem(const void* fn, size_t bytes) {
         allow_large_smem(fn);
 }
 
-// f(copy bytes, groups a CTA) for a column kernel of `groups` 32-channel groups.
-template <int WIDE = 16, class F> static void on_groups(uint64_t groups, bool aligned, F&& f) {
+// f(copy bytes, groups a CTA) for a column kernel of `groups` 32-channel
+// groups, one a CTA while they are no more than `per_sm` an SM.
+template <int WIDE = 16, class F> static void on_groups(uint64_t groups, uint64_t per_sm, bool aligned, F&& f) {
     using One  = std::integral_constant<int, 1>;
     using Many = std::integral_constant<int, cols::kManyGroups>;
-    const bool few = cols::few_groups(groups);
+    const bool few = cols::few_groups(groups, per_sm);
     if (aligned && few)
         f(std::integral_constant<int, WIDE>{}, One{});
     else if (aligned)
@@ -2095,10 +2096,7 @@ void launch_bandpass(const Dims& d, const float* samples, float* loc, float* sca
                      uint32_t* unmeasured, cudaStream_t s) {
     // level, flat flag and scale, then the clipped refinement
     const dim3 grid(grid1(d.nchans, 32), static_cast<unsigned>(d.nwin));
-    if (cols::few_groups(static_cast<uint64_t>(grid.x) * grid.y))
-        k_remedian<25><<<grid, 32 * 25, 0, s>>>(d, samples, loc, scale, inv);
-    else
-        k_remedian<8><<<grid, 32 * 8, 0, s>>>(d, samples, loc, scale, inv);
+    k_remedian<<<grid, 32 * kRemedianWarps, 0, s>>>(d, samples, loc, scale, inv);
     FB_COUNT_LAUNCH();
     auto refine = [&](auto u, auto groups) {
         constexpr int U = decltype(u)::value, G = decltype(groups)::value;
@@ -2107,7 +2105,7 @@ void launch_bandpass(const Dims& d, const float* samples, float* loc, float* sca
         const dim3 g(grid1(d.nchans, 32 * G), static_cast<unsigned>(d.nwin));
         k_bandpass_refine<U, G><<<g, 32 * (G + 1), smem, s>>>(d, samples, loc, scale, inv, unmeasured);
     };
-    on_groups(static_cast<uint64_t>(grid.x) * grid.y,
+    on_groups(static_cast<uint64_t>(grid.x) * grid.y, cols::kBandpassFew,
               d.nchans % 4 == 0 && reinterpret_cast<uintptr_t>(samples) % 16 == 0, refine);
     FB_COUNT_LAUNCH();
 }
@@ -2139,7 +2137,7 @@ void launch_moments(const Dims& d, const uint8_t* raw, const float* loc, const f
                     const uint8_t* static_mask, float clip, MomentSums* out, cudaStream_t s) {
     FB_DISPATCH(d.dtype, {
         constexpr int kWide = kBitsOf<D> >= 4 ? 16 : 4; // 32 narrower samples are no 16 bytes
-        on_groups<kWide>(grid1(d.nchans, 32) * d.nwin, aligned16(raw) && d.row_bytes % 16 == 0,
+        on_groups<kWide>(grid1(d.nchans, 32) * d.nwin, cols::kMomentsFew, aligned16(raw) && d.row_bytes % 16 == 0,
                          [&](auto u, auto groups) {
                              constexpr int U = decltype(u)::value, G = decltype(groups)::value;
                              constexpr size_t smem = G * MomentRing<D, U, G>::kBytes;
@@ -2316,7 +2314,7 @@ void launch_unpack(const Dims& d, const uint8_t* raw, float* work, cudaStream_t 
 
 void launch_welford(const Dims& d, const float* work, const double* recip, float* loc, float* scale,
                     cudaStream_t s) {
-    on_groups(grid1(d.nchans, 32) * d.nwin, aligned16(work) && d.nchans % 4 == 0, [&](auto u, auto groups) {
+    on_groups(grid1(d.nchans, 32) * d.nwin, cols::kWelfordFew, aligned16(work) && d.nchans % 4 == 0, [&](auto u, auto groups) {
         constexpr int U = decltype(u)::value, G = decltype(groups)::value;
         constexpr size_t smem = G * WorkRing<U, G>::kBytes + WorkRing<U, G>::kSideBytes;
         set_smem(reinterpret_cast<const void*>(&k_welford<U, G>), smem);
