@@ -821,12 +821,12 @@ __global__ void __launch_bounds__(kThreads, FSB == 2 ? (CH == 2048 ? 4 : 3) : (C
     //          chunks where some test may fire
     //   gmin   (halo + CH) / 4 + 4 pad: least Q of each aligned 4-column group
     //   tmin   (halo + CH) / P: least Q of each thread's P columns
-    //   nh     2 x nh_len: the next chunk's halo (Q, gmin, tmin and this
-    //          chunk's last Q, not yet rebased), by chunk parity
     //   gmax   trapezoid only: (halo + CH) / 4 + 4 pad, the greatest Q of each
-    //          group, and 2 x halo / 4 of the next chunk's halo; with a halo
-    //          wider than a chunk, which no chunk hands on, in nh's place, so
-    //          that trapezoids run as wide as boxcars do
+    //          group, and 2 x halo / 4 of the next chunk's halo
+    //   nh     2 x nh_len: the next chunk's halo (Q, gmin, tmin and this
+    //          chunk's last Q, not yet rebased), by chunk parity; a halo wider
+    //          than a chunk is not handed on, and gmax then lies in nh's room,
+    //          so that trapezoids run as wide as boxcars do
     //   bits   uint32 [nw][CH / 32]: per-width masks of the samples that fired
     //   stage  S [2][halo + CH]: the raw row segment, bulk-copied one chunk
     //          ahead (the halo columns only for the first chunk)
@@ -862,17 +862,16 @@ __global__ void __launch_bounds__(kThreads, FSB == 2 ? (CH == 2048 ? 4 : 3) : (C
     float* const gmin    = Ps + 4 + seg_cols + 4;
     float* const tmin    = gmin + seg_cols / 4 + 4;
     const int nh_len     = halo + halo / 4 + halo / P + 4;
-    float* const nh0     = tmin + seg_cols / P;
     // (the power-of-two tests are the boxcars')
     const bool trap      = !POW2 && p.trapezoid != 0;
     // A chunk's halo is the previous chunk's last `halo` columns, whose prefix
     // sums that chunk has: only the first chunk (or every chunk, for a halo
     // wider than a chunk) stages and scans its halo.
     const bool carry_halo = halo <= CH;
-    float* const nh_end   = nh0 + 2 * nh_len;
-    float* const gmax     = carry_halo ? nh_end : nh0;
+    float* const gmax     = tmin + seg_cols / P;
     float* const ghalo0   = gmax + seg_cols / 4 + 4;
-    uint32_t* const bits  = reinterpret_cast<uint32_t*>(trap && carry_halo ? ghalo0 + halo / 2 : nh_end);
+    float* const nh0      = trap && carry_halo ? ghalo0 + halo / 2 : gmax;
+    uint32_t* const bits  = reinterpret_cast<uint32_t*>(nh0 + 2 * nh_len);
     S* const stage0       = reinterpret_cast<S*>(bits + search_bits_words(nw, CH)); // buffer b at stage0 + b * seg_cols
     uint8_t* const best_w = reinterpret_cast<uint8_t*>(gmin); // across widths: CH of its 4 (halo + CH) / 4 bytes
     const int nchunks     = (p.n_valid + CH - 1) / CH;
@@ -1531,14 +1530,14 @@ void search_table(SearchSeg* segs, int n, cudaStream_t s, int32_t chunk, int32_t
     }
     const size_t es   = segs[0].fp16 ? 2 : 4;
     const size_t seg  = static_cast<size_t>(p0.halo) + chunk;
-    // Ps, gmin (+4 padding), tmin, the next chunk's halo by parity, gmax, the bit
+    // Ps, gmin (+4 padding), tmin, gmax, the next chunk's halo by parity, the bit
     // masks and the staging buffers (the kernel's layout)
     const size_t per  = static_cast<size_t>(chunk) / kThreads; // columns per thread
     const size_t nh   = static_cast<size_t>(p0.halo) + p0.halo / 4 + p0.halo / per + 4;
     // staging: two raw row segments, or (fused level step) the halo and
     // two pairs of child segments
     const size_t stage_elems = fs ? p0.halo + fsb * (2 * static_cast<size_t>(chunk) + 16 / es) : 2 * seg;
-    // gmax and its halo copies (a halo wider than a chunk: in nh's place, which
+    // gmax and its halo copies (a halo wider than a chunk: in nh's room, which
     // is larger: 2 nh > 2.5 halo > (halo + chunk) / 4 + 4)
     const size_t trap = p0.trapezoid && p0.halo <= chunk ? seg / 4 + 4 + p0.halo / 2 : 0;
     const size_t smem = sizeof(float) * ((4 + seg + 4) + (seg / 4 + 4) + seg / per + 2 * nh + trap) +
