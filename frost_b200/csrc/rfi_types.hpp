@@ -165,62 +165,6 @@ struct KadaneState {
     }
 };
 
-/** KadaneState::append with 32-bit positions (a block's samples and
- * channels stay below 2^31): the same sums, comparisons and runs, fewer
- * integer instructions in the per-sample scans; widened for storage. */
-struct KadaneState32 {
-    struct Run32 {
-        double sum;
-        int32_t start, end;
-    };
-    double total = 0.0;
-    int32_t first = 0, last = -1;
-    bool empty    = true;
-    Run32 prefix{0.0, 0, -1}, suffix{0.0, 0, -1}, best{0.0, 0, -1};
-
-    FB_HD void append(int32_t i, double u) {
-        if (empty) {
-            empty  = false;
-            first  = i;
-            prefix = {0.0, i, i - 1};
-            suffix = {0.0, i, i - 1};
-            best   = suffix;
-        }
-        last = i;
-        total += u;
-        if (total > prefix.sum) { // the prefix run always starts at `first`
-            prefix.sum = total;
-            prefix.end = i;
-        }
-        // The open (suffix) run always ends at the last position, so its end
-        // is `last` (filled in by widen) and it is empty exactly when its
-        // sum is zero (a kept run has a positive sum).
-        const double s = suffix.sum + u;
-        if (s > 0.0) {
-            if (suffix.sum == 0.0)
-                suffix.start = i;
-            suffix.sum = s;
-        } else {
-            suffix.sum   = 0.0;
-            suffix.start = i + 1;
-        }
-        if (suffix.sum > best.sum)
-            best = {suffix.sum, suffix.start, i};
-    }
-    FB_HD static Run wide(const Run32& r) { return {r.sum, r.start, r.end}; }
-    FB_HD KadaneState widen() const {
-        KadaneState k = KadaneState::make();
-        k.total       = total;
-        k.first       = first;
-        k.last        = last;
-        k.empty       = empty ? 1 : 0;
-        k.prefix      = wide(prefix);
-        k.suffix      = {suffix.sum, suffix.start, empty ? suffix.end : last};
-        k.best        = wide(best);
-        return k;
-    }
-};
-
 /** Whether a sum of floats is greater than zero, from its high word: 1 ..
  * 0x7FF00000 there means positive or +inf. Such a sum is a multiple of
  * 2^-149, so one with a zero high word is zero; a negative one has the sign
@@ -325,6 +269,20 @@ struct KadanePair32 {
     /** The state of -u (its total is 0 - total: +0 rather than -0 for a
      * zero total, as the sum of -u would be). */
     FB_HD KadaneState widen_neg(int32_t last) const { return widen(neg, 0.0 - total, last); }
+};
+
+/** KadanePair32's state of u alone, begun by its first append. */
+struct KadaneState32 {
+    KadanePair32 pair;
+    int32_t last = -1;
+
+    FB_HD void append(int32_t i, double u) {
+        if (pair.empty)
+            pair.begin(i);
+        pair.append(i, u);
+        last = i;
+    }
+    FB_HD KadaneState widen() const { return pair.widen_pos(last); }
 };
 
 /** Largest power of five not above `count` (0 for 0). */
