@@ -410,8 +410,9 @@ __global__ void __launch_bounds__(32 * kRemedianWarps)
 // after the two remedian passes: a lane per channel, a CTA per 32 channels
 // of a window. Up to six passes over the sampled rows, each one chain of
 // dependent FP64 additions in row order, streamed as rfi_columns.cuh says.
-// 1024 channels, 2 windows: 122 us (172 with a warp that copies for itself
-// and a loop the compiler orders); 4096 channels, 8 windows: 304 us.
+// 1024 channels, 2 windows: 124 us (172 with a warp that copies for itself
+// and a loop the compiler orders); 4096 channels, 8 windows: 330 us (240 so,
+// with fewer feeders in the walkers' way; 1056 with block-wide stages).
 // Each channel updates only while its own sequence of steps is still
 // running, so every channel takes the reference's steps whatever the others
 // of its warp do. A flat channel (every sampled value equal) keeps its first
@@ -580,9 +581,9 @@ __global__ void __launch_bounds__(32 * (G + 1))
 // own chain of FP64 additions, so ROLES warps of a CTA can keep them apart,
 // each reading the same columns: with ROLES = 3 (where groups are few) a
 // warp carries two or three sums (z and z^2 are formed again in each), with
-// 1 all of them. 1024 float32 channels, 2 windows of 31 250 rows: 430 us
+// 1 all of them. 1024 float32 channels x 65 536 rows, 2 windows: 425 us
 // (1611 with one warp's sums behind block-wide stages); 4096 uint8 channels,
-// 8 windows: 1410 us (1976), where 12 FP64 operations a sample bound it.
+// 8 windows: 1416 us (1976), where 12 FP64 operations a sample bound it.
 
 template <int ROLES, int ROLE, class R, class Z>
 __device__ __forceinline__ void moments_walk(const R& rows, Z&& z_of, float clip, MomentSums& out) {
@@ -1777,8 +1778,8 @@ __global__ void k_unpack(Dims d, const uint8_t* __restrict__ raw, float* __restr
 // they are many. The mean never becomes -0 (it starts at +0 and a rounded
 // sum is -0 only when both terms are), so a zero quotient (delta = +-0)
 // leaves it unchanged without a select. var's increment is added a row late,
-// in the chain's gaps. 1024 channels, 2 windows of 31 250 rows: 690 us (2276
-// before: 126 cycles a row); 4096 channels, 8 windows: 1350 us (2979).
+// in the chain's gaps. 1024 channels x 65 536 rows, 2 windows: 702 us (2276
+// before: 126 cycles a row); 4096 channels, 8 windows: 1274 us (2979).
 template <int U, int G> using WorkRing = cols::Ring<32, U, G == 1 ? 64 : 32, 4, true>;
 
 template <int U, int G>

@@ -1,7 +1,8 @@
-// Time-ordered streaming of a block's channel columns through shared memory.
+// Time-ordered streaming of a block's channel columns through shared memory,
+// for the column scan (and, of it, the cp.async helpers for the other scans).
 //
-// The order-exact statistics kernels give each thread one channel and walk
-// it in time order (their double sums must follow the reference's order).
+// The scan gives each thread one channel of a chunk and walks it in time order
+// (its double sums must follow the reference's order).
 // Read straight from HBM, each step is one byte (or word) per thread with
 // a row stride between steps: few bytes in flight and latency-bound. Here
 // the block's threads instead copy whole row segments (the block's
@@ -9,9 +10,9 @@
 // into one of two buffers, and then every thread walks its column in
 // shared memory while the other buffer fills.
 //
-// Requirements (the launchers check them and otherwise use the direct
-// kernels): the row pitch and the segment's byte offset are multiples of
-// 16 bytes.
+// Requirements (the launcher checks them and otherwise uses k_scan_cols,
+// which reads from memory): the row pitch and the segment's byte offset are
+// multiples of 16 bytes.
 #pragma once
 
 #include <cstdint>
