@@ -795,6 +795,10 @@ struct ScanRowAcc {
             sn.append(static_cast<int32_t>(c), -u);
         }
     }
+    __device__ __forceinline__ void resume() {
+        sp.resume();
+        sn.resume();
+    }
     // W32: moves the tile's integer sums into the 64-bit ones (exact: a tile
     // of at most 1024 codes of at most 8 bits sums below 2^32 even squared)
     __device__ __forceinline__ void flush() {
@@ -861,7 +865,7 @@ struct ScanRowAcc {
 // 1912 uint8 channels (pitch no multiple of 16) x 4289 rows 540 -> 99 us,
 // 1536 2-bit x 40 001: 236 -> 122, against a branch a channel and rows
 // decoded one sample at a time; 4096 x 262 144 with Kadane across frequency
-// 2550 -> 2460 (selects on the integer pipe bound it).
+// 2550 -> 2427 (selects on the integer pipe bound it).
 template <int U> constexpr int kRowStride = U == 16 ? 144 : 132;
 constexpr int kRowTileBytes = 128;
 template <int D> constexpr int kRowTiles = kBitsOf<D> == 32 ? 3 : 2;
@@ -979,6 +983,7 @@ __global__ void __launch_bounds__(kScanRows)
                         used |= in && mask[q + e] != 0 ? 1U << e : 0U;
                     }
                 }
+                acc.resume();
 #pragma unroll
                 for (int e = 0; e < kGroup; ++e) {
                     const uint32_t code = kBits == 32 ? words[e]
@@ -1002,7 +1007,7 @@ __global__ void __launch_bounds__(kScanRows)
 // constants are reloaded only when the window changes; rows are taken a few
 // at a time, without a branch where they lie in one window and the channel is
 // measured there.
-// With Kadane: 4096 uint8 channels x 262 144 rows 3150 -> 2095 us, 479 float32
+// With Kadane: 4096 uint8 channels x 262 144 rows 3150 -> 2029 us, 479 float32
 // channels x 12 734 rows 193 -> 70.
 template <bool ZDOT, bool KCHAN>
 struct ScanColAcc {

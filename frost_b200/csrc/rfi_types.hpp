@@ -165,58 +165,61 @@ struct KadaneState {
     }
 };
 
-/** Whether a sum of floats is greater than zero, from its high word: 1 ..
- * 0x7FF00000 there means positive or +inf. Such a sum is a multiple of
- * 2^-149, so one with a zero high word is zero; a negative one has the sign
- * bit set; a NaN (0 x inf of a channel whose scale has no float inverse) is
- * above +inf and, as in a comparison, not greater than zero. */
-FB_HD bool positive_sum(double s) {
+/** Whether a sum that is never -0 is less than zero, by one comparison of its
+ * high word as an integer: -inf's, 0xFFF00000, is the greatest of those that
+ * are. A NaN (0 x inf of a channel whose scale has no float inverse) is, as in
+ * a comparison, not less than zero. */
+FB_HD bool negative_sum(double s) {
 #if defined(__CUDA_ARCH__)
-    const uint32_t hi = static_cast<uint32_t>(__double2hiint(s));
+    const int32_t hi = __double2hiint(s);
 #else
     uint64_t bits;
     std::memcpy(&bits, &s, sizeof(bits));
-    const uint32_t hi = static_cast<uint32_t>(bits >> 32U);
+    const auto hi = static_cast<int32_t>(bits >> 32U);
 #endif
-    return hi - 1U < 0x7FF00000U;
+    return hi <= -0x100000;
 }
 
-/** The open (suffix) and the best run of a sequence of floats: KadaneState's
- * sums, comparisons and runs from fewer operations, without branches. The
- * open run ends at the position just appended; its start is taken at every
- * position before which it is empty (the run it starts, if any, starts
- * there). Appending 0 changes no run. */
+/** The open (suffix) and the best run of a sequence: KadaneState's sums,
+ * comparisons and runs from fewer operations, without branches, the sums
+ * kept negated (an empty run's is +0; +0 less a zero of either sign, and the
+ * difference of equal values, are +0, so no sum is -0). The open run ends at the
+ * position just appended; its start is taken at every position before which
+ * it is empty (the run it starts, if any, starts there). Appending 0 changes
+ * no run. */
 struct OpenBestRun {
-    double ssum = 0.0, bsum = 0.0;
+    double minus_open = 0.0, minus_best = 0.0;
     int32_t sstart = 0, bstart = 0, bend = -1;
-    bool open = false; // ssum > 0
+    bool open = false;
 
+    /** Before a group of appends: `open` from the sum, so that a loop over
+     * short groups need not keep it between them (rows of 3336 float32
+     * channels, 4 a group: 387 -> 357 us). */
+    FB_HD void resume() { open = negative_sum(minus_open); }
     FB_HD void append(int32_t i, double u) {
-        const double s = ssum + u;
+        const double s = minus_open - u;
         sstart         = open ? sstart : i;
-        open           = positive_sum(s);
-        ssum           = open ? s : 0.0;
-        const bool up  = ssum > bsum;
-        bsum           = up ? ssum : bsum;
+        open           = negative_sum(s);
+        minus_open     = open ? s : 0.0;
+        const bool up  = minus_open < minus_best;
+        minus_best     = up ? minus_open : minus_best;
         bstart         = up ? sstart : bstart;
         bend           = up ? i : bend;
     }
+    FB_HD Run best() const { return {0.0 - minus_best, bstart, bend}; }
 };
 
-/** The best run of KadaneState::append over a sequence of floats that is
- * never combined with another. When no run ever has a positive sum the best
- * run is empty (length 0) and reported at position 0 rather than at the
- * first position appended; callers use only a best run's length when it is
- * empty. */
-struct KadaneBest : OpenBestRun {
-    FB_HD Run best() const { return {bsum, bstart, bend}; }
-};
+/** The best run of KadaneState::append over a sequence that is never combined
+ * with another. When no run ever has a positive sum the best run is empty
+ * (length 0) and reported at position 0 rather than at the first position
+ * appended; callers use only a best run's length when it is empty. */
+struct KadaneBest : OpenBestRun {};
 
-/** The KadaneStates of a sequence u of floats and of its negation -u,
- * appended together from a known first position (`begin`): the states of -u
- * share the running total (negated: the sums of -u are the exact negations
- * of those of u) and compare it for their own best prefix; the prefix runs
- * start at the first position. */
+/** The KadaneStates of a sequence u and of its negation -u, appended together
+ * from a known first position (`begin`): the states of -u share the running
+ * total (negated: the sums of -u are the exact negations of those of u) and
+ * compare it for their own best prefix; the prefix runs start at the first
+ * position. */
 struct KadanePair32 {
     struct Side {
         double psum = 0.0;
@@ -260,8 +263,8 @@ struct KadanePair32 {
         k.last   = last;
         k.empty  = 0;
         k.prefix = {sd.psum, first, sd.pend};
-        k.suffix = {sd.run.ssum, sd.run.open ? sd.run.sstart : last + 1, last};
-        k.best   = {sd.run.bsum, sd.run.bstart, sd.run.bend};
+        k.suffix = {0.0 - sd.run.minus_open, sd.run.open ? sd.run.sstart : last + 1, last};
+        k.best   = sd.run.best();
         return k;
     }
     /** The state of u after appends up to position `last`. */
